@@ -34,7 +34,7 @@ __device__ void batch_tile(T* re, T* im, const unsigned char* __restrict__ blob,
     __syncthreads();
     if (threadIdx.x == 0) *s_loaded = range;
   }
-  run_tile<T, K, CLS>(re + R.state_off, im + R.state_off, dp->h, tb, t, sre, sim);
+  run_tile<T, K, CLS>(re + R.state_off, im + R.state_off, dp->h, tb, tile_base(dp->h, t), sre, sim);
 }
 
 template <typename T, int K>

@@ -9,11 +9,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <map>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -61,6 +63,10 @@ struct dmsim_sim {
   double* d_diag = nullptr;
   double* d_acc = nullptr;
   int* d_err = nullptr;  // set by a tensor pass whose bounded wait ran out
+  int* d_herm = nullptr; // 1: rho is Hermitian, half-range passes run on half of it (pass.h)
+  int herm_flag = 1;     // what *d_herm was last set to; -1: by the check, on the device
+  bool herm_known = true;   // rho is Hermitian by its history: |0..0><0..0| and passes that keep it so
+  bool exposed = false;     // the device pointers were handed out: rho may be written at any time
 
   std::vector<GateRec> circuit;
   std::vector<Channel> channels;  // superoperators of the circuit's noise channels
@@ -77,6 +83,10 @@ struct dmsim_sim {
   int renorm = 64;      // complex64: renormalise every renorm passes (0 = never)
   int tensor = 1;       // K = 3, 4 dense/sparse passes on the tensor cores (DMSIM_OPT_TENSOR)
   int direct1 = 1;      // 1-qubit passes on the register kernel (DMSIM_OPT_DIRECT1)
+  int hermitian = 1;    // half-range passes (DMSIM_OPT_HERMITIAN)
+  bool keeps_herm = true;   // the uploaded plan keeps a Hermitian rho Hermitian (no SRN)
+  uint32_t end_stale = 0;   // the set under which the last pass leaves the state (0: all of it up to date)
+  double half_gain_us = 0;  // what the plan's half-range passes are expected to save
   int arith = 0;        // arithmetic of the uploaded plan (kernels.h Arith)
   int64_t seed = -1;
 
@@ -97,6 +107,8 @@ void free_plan(dmsim_sim* s) {
   s->desc_bytes = 0;
   s->passes.clear();
   s->n_basic = 0;
+  s->end_stale = 0;
+  s->half_gain_us = 0;
   s->uploaded = false;
 }
 
@@ -124,6 +136,8 @@ void ensure_state(dmsim_sim* s) {
   }
   DM_CUDA(launch_set_zero_state(s->d_re, s->d_im, s->N, s->fp32, s->stream));
   DM_CUDA(cudaStreamSynchronize(s->stream));
+  s->herm_known = true;
+  s->exposed = false;
 }
 
 void check_qubits(const dmsim_sim* s, const GateRec& g) {
@@ -137,8 +151,13 @@ void check_qubits(const dmsim_sim* s, const GateRec& g) {
       if (g.qb[i] == g.qb[j]) throw DmError{DMSIM_ERR_ARG, "a gate's qubits must be distinct"};
 }
 
-// Launch the planned passes on stream st (captured or direct).
+// Launch the planned passes on stream st (captured or direct).  A timed pass
+// includes the mirror pass that it needs before it, the last one the mirror
+// that brings the whole state up to date.
 void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
+  auto mirror = [&](uint32_t from, uint32_t to, bool last) {
+    if (from) DM_CUDA(launch_mirror(s->d_re, s->d_im, (int)s->n, s->arith, from, to, last, s->d_herm, s->sms, st));
+  };
   for (size_t i = 0; i < s->passes.size(); i++) {
     PassInfo& p = s->passes[i];
     if (p.renorm) {
@@ -149,6 +168,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     }
     if (p.conv) {
       if (timed) DM_CUDA(cudaEventRecord(p.ev0, st));
+      mirror(p.stale, 0, true);
       if (p.conv == 1) DM_CUDA(launch_to_df64(s->d_re, s->d_im, s->N, p.grid, st));
       else DM_CUDA(launch_from_df64(s->d_re, s->d_im, s->N, p.grid, st));
       if (timed) DM_CUDA(cudaEventRecord(p.ev1, st));
@@ -176,8 +196,12 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.direct1 = p.direct1;
     a.q0 = p.q0;
     a.n = (int)s->n;
+    a.half = p.half ? reinterpret_cast<const HalfMap*>(static_cast<const char*>(s->d_desc) + p.half_off) : nullptr;
+    a.herm = s->d_herm;
     if (timed) DM_CUDA(cudaEventRecord(p.ev0, st));
+    if (p.stale != p.half) mirror(p.stale, p.half, false);
     DM_CUDA(launch_pass(a, st));
+    if (i + 1 == s->passes.size()) mirror(s->end_stale, 0, true);
     if (timed) DM_CUDA(cudaEventRecord(p.ev1, st));
   }
 }
@@ -235,6 +259,36 @@ std::vector<PassSpec> make_plan(dmsim_sim* s, const std::vector<Basic>& basics) 
 
 void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_basic, int arith);
 
+// What a pass takes, for the choice of half-range passes (plan_half): time
+// per entry as measured on GB300, tensor passes in whole rounds of the tiles
+// that run at once.
+HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, uint64_t ntiles) {
+  HalfCost c;
+  c.allowed = 0;
+  c.fixed_us = 2.5;
+  const double N = (double)s->N;
+  if (p.tc && s->arith == AR_FP64) {
+    c.fixed_us = 6;
+    c.slots = 2.0 * s->sms;
+    c.tiles = (double)ntiles;
+    c.tile_us = p.K == 4 ? 10.5 : 6.5;
+    return c;
+  }
+  // picoseconds per entry: memory traffic, or the multiply-adds of the pipe
+  const double bw = (p.feat.ld_frac + p.feat.st_frac) * 16 / 5.6;
+  const double rate = s->arith == AR_FP64 ? 2.0 : 0.6;  // per multiply-add
+  const int D = 1 << p.K;
+  double fma = 0;
+  if (p.cls == CLS_DENSE) fma = 2.0 * D * (p.real ? 2 : 4);
+  else if (p.cls == CLS_SPARSE) fma = 2.0 * p.feat.nnz / D * (p.real ? 2 : 4);
+  else if (p.cls == CLS_PHASE) fma = p.K > 1 ? 4.5 * p.feat.st_frac : 2;
+  else if (p.cls == CLS_SUPER) fma = 4.0 * D * D * 1.8;
+  c.slots = 1;
+  c.tiles = 1000;  // no rounding: many small tiles
+  c.tile_us = N * std::max(bw, fma * rate) * 1e-6 / c.tiles;
+  return c;
+}
+
 bool use_tensor(const dmsim_sim* s, const PassSpec& p, int arith) {
   return tc_choose(p, (int)s->n, s->tensor, arith);
 }
@@ -254,6 +308,43 @@ void upload(dmsim_sim* s) {
   upload_specs(s, make_plan(s, basics), (uint32_t)basics.size(), run_arith(s, rlin));
 }
 
+// Choose the half-range passes (pass.h) of the pass list, append their maps
+// to the descriptors and set what each pass finds stale.  Returns the new
+// size of the descriptors.
+size_t plan_half_ranges(dmsim_sim* s, const std::vector<HalfCost>& costs,
+                        const std::vector<std::array<int32_t, 10>>& geo, std::vector<unsigned char>& blob,
+                        size_t total) {
+  const double state = 2.0 * (double)s->N * (double)esize(s);  // bytes of rho
+  const double part = 0.5 * state, full = state;               // a mirror reads and writes a quarter, a half
+  const double us = 1.0 / 5.0e6;                               // at 5 TB/s
+  const std::vector<uint32_t> S = plan_half(costs, 3 + part * us, 3 + full * us, &s->half_gain_us);
+  std::map<std::pair<uint32_t, std::array<int32_t, 10>>, size_t> maps;
+  uint32_t stale = 0;
+  for (size_t i = 0; i < s->passes.size(); i++) {
+    PassInfo& p = s->passes[i];
+    p.half = S[i];
+    p.stale = stale;
+    // bytes: the half range of the pass, and the mirror before it
+    if (p.half) p.bytes *= 0.5 * (1.0 + std::ldexp(1.0, -std::min(kHalfMaxS, __builtin_popcount(p.half))));
+    if (stale != p.half && stale) p.bytes += p.half ? part : full;
+    stale = p.half;
+    if (!p.half) continue;
+    const auto key = std::make_pair(p.half, geo[i]);
+    auto it = maps.find(key);
+    if (it == maps.end()) {
+      const size_t off = (total + 15) & ~(size_t)15;
+      blob.resize(std::max(blob.size(), off + sizeof(HalfMap)));
+      build_half((int)s->n, geo[i][0], geo[i].data() + 2, geo[i][1], p.half, reinterpret_cast<HalfMap*>(blob.data() + off));
+      total = off + sizeof(HalfMap);
+      it = maps.emplace(key, off).first;
+    }
+    p.half_off = it->second;
+  }
+  s->end_stale = stale;
+  if (stale) s->passes.back().bytes += full;
+  return total;
+}
+
 // Write the descriptors of a plan to the device and capture its launches.
 void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_basic, int arith) {
   ensure_state(s);
@@ -271,6 +362,10 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
   }
   std::vector<unsigned char> blob(std::max<size_t>(total, 256));
   s->passes.clear();
+  std::vector<HalfCost> costs;                // per entry of s->passes
+  std::vector<std::array<int32_t, 10>> geo;   // its L, mhi and high target bits
+  const HalfCost whole = {0, 2.5, 0, 1, 1};
+  s->keeps_herm = true;
   const double conv_bytes = 2.0 * 2.0 * (double)s->N * 8.0;
   if (arith == AR_DF64) {
     PassInfo pi;
@@ -279,6 +374,8 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     pi.grid = (unsigned)s->sms * 8;
     pi.bytes = conv_bytes;
     s->passes.push_back(pi);
+    costs.push_back(whole);
+    geo.push_back({});
   }
   for (size_t i = 0; i < specs.size(); i++) {
     PassInfo pi;
@@ -289,8 +386,12 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       pi.grid = (unsigned)s->sms * 8;
       pi.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(pi);
+      costs.push_back(whole);
+      geo.push_back({});
+      s->keeps_herm = false;
       continue;
     }
+    if (specs[i].rlin || specs[i].ket_only) s->keeps_herm = false;
     uint64_t ntiles = 0;
     int tile = 0;
     pi.tc = tcs[i] != 0;
@@ -317,6 +418,14 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       pi.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((groups + 255) / 256, (uint64_t)s->sms * 8));
     }
     s->passes.push_back(pi);
+    const PassHeader& hd = *reinterpret_cast<const PassHeader*>(blob.data() + offs[i]);
+    HalfCost hc = half_cost(s, pi, ntiles);
+    hc.allowed = half_allowed(hd, specs[i], (int)s->n, pi.direct1);
+    costs.push_back(hc);
+    std::array<int32_t, 10> gm = {hd.L, hd.mhi};
+    for (int j = 0; j < hd.mhi; j++) gm[2 + j] = hd.hipos[j];
+    if (pi.direct1) gm = {0, 2, pi.q0, pi.q0 + (int)s->n};
+    geo.push_back(gm);
     // complex64: FP64 trace + Hermitian renormalisation every renorm passes and at the end
     if (s->fp32 && s->renorm > 0 && ((i + 1) % (size_t)s->renorm == 0 || i + 1 == specs.size())) {
       PassInfo rn;
@@ -325,6 +434,8 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       rn.grid = (unsigned)s->sms * 8;
       rn.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(rn);
+      costs.push_back(whole);
+      geo.push_back({});
     }
   }
   if (arith == AR_DF64) {
@@ -334,7 +445,12 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     pi.grid = (unsigned)s->sms * 8;
     pi.bytes = conv_bytes;
     s->passes.push_back(pi);
+    costs.push_back(whole);
+    geo.push_back({});
   }
+  // complex64 runs stay whole: their renormalisation averages the two
+  // partners' FP32 rounding errors, which a copied partner would not have
+  if (s->hermitian && s->keeps_herm && !s->fp32 && s->n >= 6) total = plan_half_ranges(s, costs, geo, blob, total);
   if (total > 0) {
     DM_CUDA(cudaMalloc(&s->d_desc, total));
     DM_CUDA(cudaMemcpyAsync(s->d_desc, blob.data(), total, cudaMemcpyHostToDevice, s->stream));
@@ -367,6 +483,25 @@ void run(dmsim_sim* s) {
   if (!s->uploaded) throw DmError{DMSIM_ERR_STATE, "run() before upload()"};
   ensure_state(s);
   const bool timed = s->record != 0;
+  bool half = false;
+  for (const PassInfo& p : s->passes) half |= p.half != 0;
+  if (half) {
+    // rho as the engine left it is Hermitian; after dmsim_set_dm or with the
+    // device pointers handed out it is compared with its transpose first
+    // (one read of the state), unless the plan would save less than that
+    const double check_us = 6 + 2.0 * (double)s->N * (double)esize(s) / 5.0e6;
+    if (s->herm_known && !s->exposed) {
+      if (s->herm_flag != 1) DM_CUDA(launch_set_flag(s->d_herm, 1, s->stream));
+      s->herm_flag = 1;
+    } else if (s->half_gain_us > check_us) {
+      DM_CUDA(launch_check_hermitian(s->d_re, s->d_im, (int)s->n, s->d_herm, s->sms, s->stream));
+      s->herm_flag = -1;
+    } else {
+      if (s->herm_flag != 0) DM_CUDA(launch_set_flag(s->d_herm, 0, s->stream));
+      s->herm_flag = 0;
+    }
+  }
+  if (!s->keeps_herm) s->herm_known = false;
   if (timed) {
     for (PassInfo& p : s->passes) {
       if (!p.ev0) DM_CUDA(cudaEventCreate(&p.ev0));
@@ -386,6 +521,7 @@ void run(dmsim_sim* s) {
     DM_CUDA(cudaMemcpy(&flag, s->d_err, sizeof flag, cudaMemcpyDeviceToHost));
     if (flag) {
       DM_CUDA(cudaMemset(s->d_err, 0, sizeof flag));
+      s->herm_known = false;
       throw DmError{DMSIM_ERR_TIMEOUT, "a tensor-core pass did not see its MMAs complete in time"};
     }
   }
@@ -436,6 +572,7 @@ void reset_dm(dmsim_sim* s) {
   ensure_state(s);
   DM_CUDA(launch_set_zero_state(s->d_re, s->d_im, s->N, s->fp32, s->stream));
   DM_CUDA(cudaStreamSynchronize(s->stream));
+  s->herm_known = true;
 }
 
 std::vector<double> host_diag(dmsim_sim* s) {
@@ -494,7 +631,9 @@ int dmsim_create(uint32_t n_qubits, uint32_t n_gpus, dmsim_handle* out) {
     DM_CUDA(cudaMalloc(&s->d_diag, s->dim * sizeof(double)));
     DM_CUDA(cudaMalloc(&s->d_acc, 8 * sizeof(double)));
     DM_CUDA(cudaMalloc(&s->d_err, 16));
-    DM_CUDA(cudaMemset(s->d_err, 0, 16));
+    const int flags[4] = {0, 1, 0, 0};
+    DM_CUDA(cudaMemcpy(s->d_err, flags, 16, cudaMemcpyHostToDevice));
+    s->d_herm = s->d_err + 1;
     // rho is allocated on first use so that complex64 can be chosen first
     // (17 qubits fit only in complex64); FP64 up to 16 qubits is allocated now
     if (n_qubits <= 16) ensure_state(s);
@@ -570,6 +709,11 @@ int dmsim_set_option(dmsim_handle s, int key, int64_t v) {
         if (s->uploaded) throw DmError{DMSIM_ERR_STATE, "set the 1-qubit kernel option before upload()"};
         s->direct1 = (int)v;
         break;
+      case DMSIM_OPT_HERMITIAN:
+        if (v != 0 && v != 1) throw DmError{DMSIM_ERR_ARG, "hermitian must be 0 or 1"};
+        if (s->uploaded) throw DmError{DMSIM_ERR_STATE, "set the half-range option before upload()"};
+        s->hermitian = (int)v;
+        break;
       case DMSIM_OPT_TENSOR:
         if (v < 0 || v > 2) throw DmError{DMSIM_ERR_ARG, "tensor must be 0, 1 or 2"};
         if (s->uploaded) throw DmError{DMSIM_ERR_STATE, "set the tensor-core option before upload()"};
@@ -602,6 +746,7 @@ int dmsim_get_option(dmsim_handle s, int key, int64_t* v) {
       case DMSIM_OPT_PLAIN_ARITH: *v = s->plain_arith; break;
       case DMSIM_OPT_TENSOR: *v = s->tensor; break;
       case DMSIM_OPT_DIRECT1: *v = s->direct1; break;
+      case DMSIM_OPT_HERMITIAN: *v = s->hermitian; break;
       default: throw DmError{DMSIM_ERR_ARG, "unknown option"};
     }
   });
@@ -822,6 +967,7 @@ int dmsim_set_dm(dmsim_handle s, const double* re, const double* im) {
   DM_TRY(s, {
     if (!re || !im) throw DmError{DMSIM_ERR_ARG, "null buffer"};
     ensure_state(s);
+    s->herm_known = false;
     if (!s->fp32) {
       DM_CUDA(cudaMemcpyAsync(s->d_re, re, s->N * 8, cudaMemcpyHostToDevice, s->stream));
       DM_CUDA(cudaMemcpyAsync(s->d_im, im, s->N * 8, cudaMemcpyHostToDevice, s->stream));
@@ -1002,6 +1148,7 @@ int dmsim_pure_metrics_noalloc(dmsim_handle s, const double* psi_re, const doubl
 int dmsim_device_state(dmsim_handle s, void** re, void** im) {
   DM_TRY(s, {
     ensure_state(s);
+    s->exposed = true;
     if (re) *re = s->d_re;
     if (im) *im = s->d_im;
   });
@@ -1118,6 +1265,7 @@ int dmsim_cost_collect(uint32_t n, uint32_t n_circuits, uint32_t gates, uint64_t
   try {
     h->record = 1;
     h->graph_on = 0;
+    h->hermitian = 0;  // the model predicts passes over the whole state
     const int widths[] = {1, 2, 3, 4};
     const int caps[] = {kMaxD, 8, 4, 2};
     for (uint32_t c = 0; c < n_circuits; c++) {

@@ -24,6 +24,9 @@ struct PassInfo {
   bool real;            // real operator (kernels_real.cu for K <= 2)
   bool direct1;         // 1-qubit pass on the register kernel (kernels_k1.cu)
   int q0;               // first target qubit
+  uint32_t half;        // half-range pass: its qubit set S (0: the whole state)
+  uint32_t stale;       // the set under which the state is up to date before the pass: a mirror pass goes first
+  size_t half_off;      // byte offset of its HalfMap in the device blob
   PassFeatures feat;
   cudaEvent_t ev0, ev1; // per-pass timing (record mode)
 };

@@ -187,6 +187,110 @@ cudaError_t launch_conj_transpose(void* re, void* im, int n, bool fp32, unsigned
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------- half-range passes
+// Between half-range passes over different qubit sets (pass.h) the entries
+// that the last set left stale and the next one needs are the conjugates of
+// their transposes: A[c*dim + r] = conj(A[r*dim + c]) where r & from > c & from
+// and r & to <= c & to (to = 0: every stale one).  About half of the stale
+// entries, a quarter of the state read and a quarter written.  The last mirror
+// of a run (`last`) fills every stale entry and makes the pairs that were both
+// computed exactly Hermitian too, so that the state passes the check below
+// again.  32 x 32 entry blocks through shared memory, both sides coalesced;
+// blocks that the sets' bits >= 5 rule out are skipped.  Entries are moved as
+// bits, `neg` is their sign bits (two in a double-float entry).
+__global__ void __launch_bounds__(256) k_mirror(uint64_t* __restrict__ re, uint64_t* __restrict__ im, int n,
+                                                uint32_t from, uint32_t to, int last, uint64_t neg,
+                                                const int* __restrict__ herm) {
+  using U = uint64_t;
+  constexpr int TS = 32;
+  __shared__ U s_re[TS][TS + 1], s_im[TS][TS + 1];
+  if (!*herm) return;
+  const uint64_t dim = 1ull << n;
+  const uint32_t nt = (uint32_t)(dim / TS);
+  const uint32_t hf = from & ~(TS - 1u), ht = to & ~(TS - 1u);
+  const uint32_t tx = threadIdx.x & 31, ty0 = threadIdx.x >> 5;
+  for (uint64_t p = blockIdx.x; p < (uint64_t)nt * nt; p += gridDim.x) {
+    const uint32_t R = (uint32_t)(p & (nt - 1)) * TS, C = (uint32_t)(p >> (n - 5)) * TS;
+    if ((R & hf) < (C & hf) || (R & ht) > (C & ht)) continue;                 // nothing stale, nothing needed
+    if ((from & (TS - 1u)) == 0 && (R & hf) == (C & hf) && !(last && R >= C)) continue;  // all ties
+    for (uint32_t ty = ty0; ty < TS; ty += 8) {
+      const uint64_t i = (uint64_t)(R + ty) * dim + C + tx;  // rho[C + tx][R + ty]
+      s_re[ty][tx] = re[i];
+      s_im[ty][tx] = im[i];
+    }
+    __syncthreads();
+    for (uint32_t ty = ty0; ty < TS; ty += 8) {
+      const uint32_t r = R + tx, c = C + ty;
+      const uint32_t rf = r & from, cf = c & from;
+      const bool stale = rf > cf && (r & to) <= (c & to);
+      const uint64_t i = (uint64_t)c * dim + r;
+      if (stale || (last && rf == cf && r > c)) {
+        re[i] = s_re[tx][ty];
+        im[i] = s_im[tx][ty] ^ neg;
+      } else if (last && r == c) {
+        im[i] = 0;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+cudaError_t launch_mirror(void* re, void* im, int n, int arith, uint32_t from, uint32_t to, bool last,
+                          const int* herm, int sms, cudaStream_t s) {
+  if (n < 5 || arith == AR_FP32) return cudaErrorInvalidValue;
+  // an odd grid: a block's tiles then run through all the residues that the sets' bits decide by
+  const uint64_t nt = 1ull << (n - 5);
+  const unsigned grid = (unsigned)std::min<uint64_t>(nt * nt, (uint64_t)sms * 8 - 1);
+  k_mirror<<<grid, 256, 0, s>>>((uint64_t*)re, (uint64_t*)im, n, from, to, last,
+                                arith == AR_DF64 ? 0x8000000080000000ull : 0x8000000000000000ull, herm);
+  return cudaGetLastError();
+}
+
+// rho may have been written from outside (dmsim_set_dm, the device pointers),
+// so a run that would use half-range passes on it first compares every entry
+// with its transpose, bit by value: one read of the state.  A NaN fails.
+__global__ void __launch_bounds__(256) k_check_hermitian(const double* __restrict__ re, const double* __restrict__ im,
+                                                         int n, int* __restrict__ herm) {
+  constexpr int TS = 32;
+  __shared__ double s_re[TS][TS + 1], s_im[TS][TS + 1];
+  const uint64_t dim = 1ull << n;
+  const uint32_t nt = (uint32_t)(dim / TS);
+  const uint32_t tx = threadIdx.x & 31, ty0 = threadIdx.x >> 5;
+  bool ok = true;
+  for (uint64_t p = blockIdx.x; p < (uint64_t)nt * nt; p += gridDim.x) {
+    const uint32_t R = (uint32_t)(p & (nt - 1)) * TS, C = (uint32_t)(p >> (n - 5)) * TS;
+    if (R > C) continue;
+    for (uint32_t ty = ty0; ty < TS; ty += 8) {
+      const uint64_t i = (uint64_t)(R + ty) * dim + C + tx;
+      s_re[ty][tx] = re[i];
+      s_im[ty][tx] = im[i];
+    }
+    __syncthreads();
+    for (uint32_t ty = ty0; ty < TS; ty += 8) {
+      const uint64_t i = (uint64_t)(C + ty) * dim + R + tx;
+      ok = ok && re[i] == s_re[tx][ty] && im[i] == -s_im[tx][ty];
+    }
+    __syncthreads();
+  }
+  if (!ok) *herm = 0;  // every writer writes the same value
+}
+
+__global__ void k_set_flag(int* f, int v) { *f = v; }
+
+cudaError_t launch_check_hermitian(const void* re, const void* im, int n, int* herm, int sms, cudaStream_t s) {
+  if (n < 5) return cudaErrorInvalidValue;
+  const uint64_t nt = 1ull << (n - 5);
+  const unsigned grid = (unsigned)std::min<uint64_t>(nt * nt, (uint64_t)sms * 8 - 1);
+  k_set_flag<<<1, 1, 0, s>>>(herm, 1);
+  k_check_hermitian<<<grid, 256, 0, s>>>((const double*)re, (const double*)im, n, herm);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_set_flag(int* flag, int value, cudaStream_t s) {
+  k_set_flag<<<1, 1, 0, s>>>(flag, value);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- renormalisation
 // complex64 mode: every R passes, trace(rho) is summed in FP64 and rho is made
 // Hermitian with unit trace, A <- (A + A^dagger) / (2 tr), each entry in the

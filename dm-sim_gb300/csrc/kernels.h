@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pass.h"
+
 namespace dmg {
 
 // Arithmetic of a pass: the state's element type.
@@ -23,6 +25,8 @@ struct LaunchArgs {
   int* err;            // device flag set to 1 when a bounded wait of a tensor pass runs out
   bool direct1;        // 1-qubit pass run by the register kernel (kernels_k1.cu)
   int q0, n;           // its qubit and the state's qubit count
+  const HalfMap* half; // device map of a half-range pass (pass.h), else null
+  const int* herm;     // device flag: half-range passes run on the half range (the state is Hermitian)
 };
 
 // Launch one pass on stream s.
@@ -48,6 +52,13 @@ cudaError_t launch_to_df64(void* re, void* im, uint64_t N, unsigned grid, cudaSt
 cudaError_t launch_from_df64(void* re, void* im, uint64_t N, unsigned grid, cudaStream_t s);
 // In place A'[x*2^n + y] = conj(A[y*2^n + x]) (the reference's adjoint stage)
 cudaError_t launch_conj_transpose(void* re, void* im, int n, bool fp32, unsigned grid, cudaStream_t s);
+// Entries stale under `from` that `to` needs (0: every one) <- conj of their
+// transposes, if *herm.  last: also make the ties exactly Hermitian.
+cudaError_t launch_mirror(void* re, void* im, int n, int arith, uint32_t from, uint32_t to, bool last,
+                          const int* herm, int sms, cudaStream_t s);
+// *herm <- 1 if rho (FP64 entries) equals its conjugate transpose exactly, else 0
+cudaError_t launch_check_hermitian(const void* re, const void* im, int n, int* herm, int sms, cudaStream_t s);
+cudaError_t launch_set_flag(int* flag, int value, cudaStream_t s);
 // rho <- (rho + rho^dagger) / (2 trace), trace summed in FP64 into d_trace
 cudaError_t launch_renormalise(void* re, void* im, int n, bool fp32, double* d_trace, unsigned grid, cudaStream_t s);
 // rho <- |0..0><0..0|

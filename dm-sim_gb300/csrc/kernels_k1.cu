@@ -19,7 +19,8 @@ namespace {
 
 template <typename T, int CLS_>
 __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict__ im,
-                                               const PassDesc<1>* __restrict__ dp, int q, int n) {
+                                               const PassDesc<1>* __restrict__ dp, int q, int n,
+                                               const HalfMap* __restrict__ half, const int* __restrict__ herm) {
   constexpr int CLS = base_class(CLS_);
   constexpr bool RE = real_class(CLS_);
   constexpr bool kMono = CLS == CLS_MOVE || CLS == CLS_SIGNED || CLS == CLS_PHASE;
@@ -59,12 +60,18 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
     need[e] = nd;
   }
 
-  const uint64_t ngroups = 1ull << (2 * n - 2);
+  const HalfMap* hm = half && *herm ? half : nullptr;  // the half range of the groups, if any
+  const uint64_t ngroups = hm ? hm->count : 1ull << (2 * n - 2);
   const uint64_t mq = 1ull << q, mb = 1ull << (q + n);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += stride) {
-    uint64_t i = ((g >> q) << (q + 1)) | (g & (mq - 1));
-    i = ((i >> (q + n)) << (q + n + 1)) | (i & (mb - 1));
+    uint64_t i;
+    if (hm) {
+      i = half_base(*hm, g, 0);
+    } else {
+      i = ((g >> q) << (q + 1)) | (g & (mq - 1));
+      i = ((i >> (q + n)) << (q + n + 1)) | (i & (mb - 1));
+    }
     uint64_t idx[4];
     idx[0] = i;
     idx[1] = i + mq;
@@ -151,7 +158,7 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
 template <typename T, int CLS_>
 cudaError_t launch1(const LaunchArgs& a, cudaStream_t s) {
   k_pass1<T, CLS_><<<a.grid, 256, 0, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                          static_cast<const PassDesc<1>*>(a.desc), a.q0, a.n);
+                                          static_cast<const PassDesc<1>*>(a.desc), a.q0, a.n, a.half, a.herm);
   return cudaGetLastError();
 }
 

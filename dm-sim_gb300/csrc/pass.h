@@ -94,6 +94,59 @@ struct PassDesc {
   PassOp<K> op;
 };
 
+// ---- half-range passes
+// rho is Hermitian through a whole run (U rho U^dagger and every channel keep
+// it so), so a pass may leave one entry of every pair rho[r][c], rho[c][r]
+// stale.  S is a set of qubits that the pass does not target: all the entries
+// of a tile have the same ket bits and the same bra bits on S, so the tile as
+// a whole has r & S <= c & S or it has not, and only the tiles that have are
+// enumerated -- (1 + 2^-|S|) / 2 of them.  Consecutive passes share one S as
+// long as none targets a qubit of it; between two different sets, and at the
+// end of the run, a mirror pass copies the conjugate transpose into the stale
+// entries that the next set needs.  FP64 and double-float runs only.
+// Measured, whole against half with the mirrors: 14 qubits, 200 mixed gates
+// fused, 460 -> 266 ms; 13 qubits gate by gate 264 -> 145 ms; 10 qubits fused
+// (state in L2) 0.63 -> 0.52 ms.
+//
+// Tiles (or, for the register kernel, groups of four entries) are numbered
+// k = pair << mlog | m: `pair` counts the ordered pairs I <= J of S values,
+// m the remaining bits.  The global index of the first entry is m << L with
+// zero gaps inserted at the S bits and at the high target bits, plus koff[I]
+// and boff[J].
+constexpr int kHalfMaxS = 5;  // 33/64 of the tiles
+struct HalfMap {
+  uint32_t mask;             // S
+  int32_t s;                 // |S|, 1..kHalfMaxS
+  int32_t mlog;
+  int32_t ngap;
+  uint64_t count;            // tiles (groups) of the half range
+  uint32_t inv;              // ceil(2^16 / (2^s + 1)): the pair's row without a division
+  uint8_t pos[20], width[20];// gaps, ascending: `width` zero bits at `pos`
+  uint64_t koff[1 << kHalfMaxS], boff[1 << kHalfMaxS];
+};
+
+// The p-th pair I <= J < B = 2^s: rows I and B-1-I of the triangle together
+// hold B + 1 pairs.
+DMG_HD inline void half_pair(uint32_t p, int s, uint32_t inv, uint32_t& I, uint32_t& J) {
+  const uint32_t B = 1u << s;
+  const uint32_t i = (p * inv) >> 16;
+  const uint32_t j = p - i * (B + 1);
+  const bool lower = j < B - i;
+  I = lower ? i : B - 1 - i;
+  J = lower ? i + j : j - 1;
+}
+// Global index of the first entry of tile k of the half range.
+DMG_HD inline uint64_t half_base(const HalfMap& hm, uint64_t k, int L) {
+  uint32_t I, J;
+  half_pair((uint32_t)(k >> hm.mlog), hm.s, hm.inv, I, J);
+  uint64_t x = (k & ((1ull << hm.mlog) - 1)) << L;
+  for (int g = 0; g < hm.ngap; g++) {
+    const int p = hm.pos[g];
+    x = ((x >> p) << (p + hm.width[g])) | (x & ((1ull << p) - 1));
+  }
+  return x | hm.koff[I] | hm.boff[J];
+}
+
 // ---- tensor-core passes (K = 3, 4; double-float or complex64 state)
 // The ket step multiplies each tile column x (2^K complex entries, as 2R
 // reals [re; im]) by the real embedding W = [[Ur, -Ui], [Ui, Ur]] (R x R,

@@ -334,6 +334,11 @@ __device__ __forceinline__ uint64_t tile_base(const PassHeader& h, uint64_t t) {
   return base;
 }
 
+// Global index of the first entry of tile t: of the half range, or of all tiles.
+__device__ __forceinline__ uint64_t tile_base(const PassHeader& h, const HalfMap* __restrict__ hm, uint64_t t) {
+  return hm ? half_base(*hm, t, h.L) : tile_base(h, t);
+}
+
 // Register staging of one tile's loads: thread tid holds entry pairs
 // tid + 256 i (i < P) -- the next tile's loads are issued before the current
 // tile is transformed, so their latency hides behind its arithmetic.
@@ -379,17 +384,16 @@ __device__ void tile_body(T* __restrict__ re, T* __restrict__ im, const PassHead
                           int lf);
 __device__ __forceinline__ int free_offset(const PassHeader& h);
 
-// One tile t of the pass on the state (re, im).  All threads of the block;
+// One tile of the pass, at global index `base`, on the state (re, im).  All threads of the block;
 // sre/sim hold G * 4^K entries each.  Ends synchronised.
 template <typename T, int K, int CLS>
 __device__ void run_tile(T* __restrict__ re, T* __restrict__ im, const PassHeader& h,
-                         const PassTables<T, K, CLS>& tb, uint64_t t, T* __restrict__ sre, T* __restrict__ sim) {
+                         const PassTables<T, K, CLS>& tb, uint64_t base, T* __restrict__ sre, T* __restrict__ sim) {
   using T2 = typename Vec2<T>::type;
   const int tid = threadIdx.x;
   const int L = h.L;
   const int tile = (1 << h.g) * (1 << K) * (1 << K);
   const int runlen = 1 << L;
-  const uint64_t base = tile_base(h, t);
   // ---- load touched runs (pairs of entries; runs are >= 2 long)
   for (int e2 = tid; e2 < (tile >> 1); e2 += blockDim.x) {
     const int e = e2 << 1;

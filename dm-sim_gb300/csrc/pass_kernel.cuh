@@ -16,10 +16,13 @@ namespace dmg {
 // then grid-strides over the tiles.
 template <typename T, int K, int CLS>
 __global__ void __launch_bounds__(kThreads) k_pass(T* __restrict__ re, T* __restrict__ im,
-                                                   const PassDesc<K>* __restrict__ dp) {
+                                                   const PassDesc<K>* __restrict__ dp,
+                                                   const HalfMap* __restrict__ half, const int* __restrict__ herm) {
   constexpr int D = 1 << K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const PassHeader& h = dp->h;
+  const HalfMap* hm = half && *herm ? half : nullptr;
+  const uint64_t ntiles = hm ? hm->count : h.ntiles;
   const int tile = (1 << h.g) * D * D;
   T* sre = reinterpret_cast<T*>(smem_raw);
   T* sim = sre + tile;
@@ -32,24 +35,24 @@ __global__ void __launch_bounds__(kThreads) k_pass(T* __restrict__ re, T* __rest
   if constexpr ((K >= 1 && K <= 2) || (std::is_same<T, float>::value && base_class(CLS) == CLS_DENSE)) {
     if (tile == 2 * kThreads * P) {
       uint64_t t = blockIdx.x;
-      if (t >= h.ntiles) return;
+      if (t >= ntiles) return;
       TileRegs<T, P> x;
       const int lf = free_offset(h);
-      uint64_t base = tile_base(h, t);
+      uint64_t base = tile_base(h, hm, t);
       load_regs<T, K, CLS, P>(re, im, h, tb, base, x);
-      for (; t < h.ntiles; t += gridDim.x) {
+      for (; t < ntiles; t += gridDim.x) {
         regs_to_smem<T, K, CLS, P>(h, tb, x, sre, sim);
         __syncthreads();
         const uint64_t tn = t + gridDim.x;
-        const uint64_t base_n = tn < h.ntiles ? tile_base(h, tn) : 0;
-        if (tn < h.ntiles) load_regs<T, K, CLS, P>(re, im, h, tb, base_n, x);
+        const uint64_t base_n = tn < ntiles ? tile_base(h, hm, tn) : 0;
+        if (tn < ntiles) load_regs<T, K, CLS, P>(re, im, h, tb, base_n, x);
         tile_body<T, K, CLS>(re, im, h, tb, base, sre, sim, lf);
         base = base_n;
       }
       return;
     }
   }
-  for (uint64_t t = blockIdx.x; t < h.ntiles; t += gridDim.x) run_tile<T, K, CLS>(re, im, h, tb, t, sre, sim);
+  for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) run_tile<T, K, CLS>(re, im, h, tb, tile_base(h, hm, t), sre, sim);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -78,7 +81,7 @@ inline cudaError_t launch_one(const LaunchArgs& a, cudaStream_t s) {
     configured = 1;
   }
   k_pass<T, K, CLS><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                                   static_cast<const PassDesc<K>*>(a.desc));
+                                                   static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
   return cudaGetLastError();
 }
 

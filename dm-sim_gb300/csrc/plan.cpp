@@ -720,6 +720,125 @@ uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uin
   return build_tc_k<4>(p, n, static_cast<TcDesc<4>*>(out), f, ntiles, tile_entries, slices, per_entry);
 }
 
+// ---------------------------------------------------------------- half-range passes
+uint32_t half_allowed(const PassHeader& h, const PassSpec& p, int n, bool direct1) {
+  if (p.transpose || p.rlin || p.ket_only) return 0;
+  const int lo = direct1 ? 5 : h.L;
+  uint32_t m = 0;
+  for (int q = lo; q < n; q++) m |= 1u << q;
+  for (int i = 0; i < p.K; i++) m &= ~(1u << p.q[i]);
+  return m;
+}
+
+void build_half(int n, int L, const int32_t* hipos, int mhi, uint32_t mask, HalfMap* out) {
+  std::memset(out, 0, sizeof *out);
+  std::vector<int> S, gaps(hipos, hipos + mhi);
+  for (int q = 0; q < n; q++)
+    if ((mask >> q) & 1) S.push_back(q);
+  for (int q : S) {
+    gaps.push_back(q);
+    gaps.push_back(q + n);
+  }
+  std::sort(gaps.begin(), gaps.end());
+  for (int p : gaps) {
+    const int g = out->ngap - 1;
+    if (g >= 0 && out->pos[g] + out->width[g] == p) out->width[g]++;
+    else {
+      out->pos[out->ngap] = (uint8_t)p;
+      out->width[out->ngap++] = 1;
+    }
+  }
+  const int s = (int)S.size();
+  const uint32_t B = 1u << s;
+  out->mask = mask;
+  out->s = s;
+  out->mlog = 2 * n - L - mhi - 2 * s;
+  out->count = (uint64_t)(B * (B + 1) / 2) << out->mlog;
+  out->inv = (65536 + B) / (B + 1);
+  for (uint32_t v = 0; v < B; v++)
+    for (int i = 0; i < s; i++) {
+      out->koff[v] |= (uint64_t)((v >> i) & 1) << S[i];
+      out->boff[v] |= (uint64_t)((v >> i) & 1) << (S[i] + n);
+    }
+}
+
+namespace {
+uint32_t top_bits(uint32_t m, int count) {  // the highest `count` bits of m
+  uint32_t r = 0;
+  for (int q = 31; q >= 0 && count > 0; q--)
+    if ((m >> q) & 1) {
+      r |= 1u << q;
+      count--;
+    }
+  return r;
+}
+double pass_us(const HalfCost& c, int s) {
+  const double f = s == 0 ? 1.0 : 0.5 * (1.0 + std::ldexp(1.0, -s));
+  return c.fixed_us + c.tile_us * std::max(1.0, std::ceil(c.tiles * f / c.slots));
+}
+int count_bits(uint32_t m) {
+  int c = 0;
+  for (; m; m &= m - 1) c++;
+  return std::min(c, kHalfMaxS);
+}
+}  // namespace
+
+std::vector<uint32_t> plan_half(const std::vector<HalfCost>& passes, double part_us, double full_us, double* gain_us) {
+  const int m = (int)passes.size();
+  constexpr int kReach = 256;  // passes of one stretch, at most
+  const double inf = 1e300;
+  // best time of the first i passes when the whole state is up to date (f) or
+  // half of it is (h), and the pass that the last stretch began with (the
+  // pass itself, marked, when it is a full one)
+  std::vector<double> f(m + 1, inf), h(m + 1, inf);
+  std::vector<int> from(m + 1, -1);
+  std::vector<char> from_half(m + 1, 0), full_from_half(m + 1, 0);
+  f[0] = 0;
+  double all = 0;
+  for (int i = 0; i < m; i++) {
+    const double t = pass_us(passes[i], 0);
+    all += t;
+    const double a = f[i] + t, b = h[i] + full_us + t;
+    if (std::min(a, b) < f[i + 1]) {
+      f[i + 1] = std::min(a, b);
+      full_from_half[i + 1] = b < a;
+    }
+    const double start = std::min(f[i], h[i] + part_us);
+    const bool start_half = h[i] + part_us < f[i];
+    uint32_t S = ~0u;
+    // per |S| the time of the stretch so far
+    double sum[kHalfMaxS + 1] = {0};
+    for (int j = i; j < m && j < i + kReach; j++) {
+      S &= passes[j].allowed;
+      if (S == 0) break;
+      for (int s = 1; s <= kHalfMaxS; s++) sum[s] += pass_us(passes[j], s);
+      const double c = start + sum[count_bits(S)];
+      if (c < h[j + 1]) {
+        h[j + 1] = c;
+        from[j + 1] = i;
+        from_half[j + 1] = start_half;
+      }
+    }
+  }
+  std::vector<uint32_t> out(m, 0);
+  const bool end_half = h[m] + full_us < f[m];
+  if (gain_us) *gain_us = std::max(0.0, all - std::min(f[m], h[m] + full_us));
+  for (int i = m, half = end_half; i > 0;) {
+    if (!half) {
+      half = full_from_half[i];
+      i--;
+      continue;
+    }
+    const int b = from[i];
+    uint32_t S = ~0u;
+    for (int j = b; j < i; j++) S &= passes[j].allowed;
+    for (int j = b; j < i; j++) out[j] = top_bits(S, kHalfMaxS);
+    half = from_half[i];
+    i = b;
+  }
+  return out;
+}
+
 bool tc_eligible(const PassSpec& p, int n) {
   if (p.transpose || p.rlin || p.super) return false;
   if (p.K != 3 && p.K != 4) return false;

@@ -81,6 +81,26 @@ size_t tc_desc_bytes(int K, int arith = 2);
 // slices = false: geometry and features only (the planner's scoring).
 uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uint64_t* ntiles, int* tile_entries,
                        bool slices = true, int arith = 2);
+// ---- half-range passes (pass.h)
+// The qubits that a pass's tiles have one ket and one bra value of: the set S
+// of a half-range pass is drawn from them.  Tiled passes: not targets, and
+// their ket bits at or above the tile's contiguous run; the register kernel:
+// not the target, and bit 5 or above (its warps stay coalesced).
+uint32_t half_allowed(const PassHeader& h, const PassSpec& p, int n, bool direct1);
+// The map of a pass with run length 2^L and high target bits hipos[0..mhi-1].
+void build_half(int n, int L, const int32_t* hipos, int mhi, uint32_t mask, HalfMap* out);
+// What a pass is expected to take, from its share of the tiles.
+struct HalfCost {
+  uint32_t allowed;    // half_allowed; 0: the whole state (also conversions and renormalisations)
+  double fixed_us;     // whatever the range
+  double tile_us;      // per round of `slots` tiles ...
+  double tiles, slots; // ... of which a full pass has `tiles`
+};
+// The set S of every pass (0: the whole state): the cheapest cut of the
+// sequence into stretches that share a set (at most kHalfMaxS qubits, the
+// highest), each paying a mirror pass at its end -- part_us between two
+// sets, full_us when the whole state is needed next or the run ends.
+std::vector<uint32_t> plan_half(const std::vector<HalfCost>& passes, double part_us, double full_us, double* gain_us);
 // x rounded to the nearest BF16 value, as a float.
 float bf16_round(float x);
 // The 7 balanced base-256 digits of an integer |t| <= 2^55 (digit 0 the most

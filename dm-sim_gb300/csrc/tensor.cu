@@ -305,7 +305,9 @@ template <> struct TcMinBlocks<float> { static constexpr int value = 3; };
 
 template <int K, typename T>
 __global__ void __launch_bounds__(kThreads, TcMinBlocks<T>::value) k_pass_tc(T* __restrict__ re, T* __restrict__ im,
-                                                         const TcDesc<K>* __restrict__ dp, int* __restrict__ err) {
+                                                         const TcDesc<K>* __restrict__ dp, int* __restrict__ err,
+                                                         const HalfMap* __restrict__ hmap,
+                                                         const int* __restrict__ herm) {
   using SH = TcShape<K, T>;
   using T2 = typename Vec2<T>::type;
   constexpr int D = SH::D, S = SH::S;
@@ -378,9 +380,11 @@ __global__ void __launch_bounds__(kThreads, TcMinBlocks<T>::value) k_pass_tc(T* 
   T* nre = reinterpret_cast<T*>(sA);
   T* nim = nre + SH::TILE;
   constexpr int PAIRS = SH::TILE / 2 / kThreads;
+  const HalfMap* hm = hmap && *herm ? hmap : nullptr;  // the half range of the tiles, if any
+  const uint64_t ntiles = hm ? hm->count : h.ntiles;
   uint64_t t = blockIdx.x;
-  if (t < h.ntiles) {
-    const uint64_t base = tile_base(h, t);
+  if (t < ntiles) {
+    const uint64_t base = tile_base(h, hm, t);
     for (int e2 = tid; e2 < (SH::TILE >> 1); e2 += blockDim.x) {
       const int e = e2 << 1;
       const int run = e >> L;
@@ -389,12 +393,12 @@ __global__ void __launch_bounds__(kThreads, TcMinBlocks<T>::value) k_pass_tc(T* 
       *reinterpret_cast<T2*>(sim + e) = ld2<T>(im + ga);
     }
   }
-  for (; t < h.ntiles; t += gridDim.x) {
+  for (; t < ntiles; t += gridDim.x) {
     __syncthreads();
-    const uint64_t base = tile_base(h, t);
+    const uint64_t base = tile_base(h, hm, t);
     const uint64_t tn = t + gridDim.x;
-    const bool has_next = tn < h.ntiles;
-    const uint64_t base_n = has_next ? tile_base(h, tn) : 0;
+    const bool has_next = tn < ntiles;
+    const uint64_t base_n = has_next ? tile_base(h, hm, tn) : 0;
     auto nothing = [] {};
     auto prefetch = [&] {
       if (!has_next) return;
@@ -463,7 +467,7 @@ static cudaError_t launch_tc_k(const LaunchArgs& a, cudaStream_t s) {
     configured = 1;
   }
   k_pass_tc<K, T><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                                  static_cast<const TcDesc<K>*>(a.desc), a.err);
+                                                  static_cast<const TcDesc<K>*>(a.desc), a.err, a.half, a.herm);
   return cudaGetLastError();
 }
 

@@ -96,6 +96,7 @@ struct T64Group {
   static constexpr int D = 1 << K;
   uint64_t full;          // the group's tile loads
   uint64_t mma;           // the group's ket and bra commits, alternating
+  uint64_t nbase;         // global index of the group's next tile
   uint32_t brmax[128];    // per bra column: magnitude key of the ket outputs
   int colEt[D][128 / D];  // biased exponent of ket column (b, f)'s grid, at [b][f]
 };
@@ -266,7 +267,7 @@ __device__ __forceinline__ void issue_step(const unsigned char* sA, const unsign
 template <int K>
 __global__ void __launch_bounds__(kT64Threads, 1)
     k_pass_tc64(uint64_t* __restrict__ re, uint64_t* __restrict__ im, const TcDesc64<K>* __restrict__ dp,
-                int* __restrict__ err) {
+                int* __restrict__ err, const HalfMap* __restrict__ hmap, const int* __restrict__ herm) {
   using S = T64<K>;
   constexpr int D = S::D, R = S::R, G = S::G, TILE = S::TILE, ASTR = S::ASTR;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -372,7 +373,8 @@ __global__ void __launch_bounds__(kT64Threads, 1)
   // buf[basec + tb.pk[cc NV + i]] (the offsets read from shared memory, a
   // broadcast per 8 lanes, to keep the 64-register budget)
   const int basec = hc * ASTR + tb.pb[rc] + piece_off(free_off(fc));
-  const uint64_t ntiles = h.ntiles, gstep = 2 * (uint64_t)gridDim.x;
+  const HalfMap* hm = hmap && *herm ? hmap : nullptr;  // the half range of the tiles, if any
+  const uint64_t ntiles = hm ? hm->count : h.ntiles, gstep = 2 * (uint64_t)gridDim.x;
   const int runlen = 1 << L, lgp = L < 4 ? L : 4, npieces = (2 * TILE) >> lgp;
   // The ket step's exact integer outputs Y(a, b) of column (b, ff) replace
   // the tile in its buffer, at [hh][a][b ^ (a & 1)][ff]: the ket step writes,
@@ -380,6 +382,7 @@ __global__ void __launch_bounds__(kT64Threads, 1)
   // b, columns a of both parities -- both free of bank conflicts.
   auto yoff = [&](int hh, int a, int b, int ff) { return hh * ASTR + (a * D + (b ^ (a & 1))) * G + ff; };
   auto tile_base_s = [&](uint64_t t) {  // tile_base from the staged positions
+    if (hm) return half_base(*hm, t, L);
     uint64_t base = t << L;
     for (int j = 0; j < mhi; j++) {
       const int p = tb.hipos[j];
@@ -460,6 +463,10 @@ __global__ void __launch_bounds__(kT64Threads, 1)
       tc::mma_commit(&gp.mma);
     }
     pendm = 1;
+    const uint64_t tn = t + gstep;
+    // one thread finds the group's next tile while the products run (every
+    // thread reads it in step 5, two barriers on)
+    if (gtid == kT64GroupThreads - 1 && tn < ntiles) gp.nbase = tile_base_s(tn);
 
     // ---- 3: ket outputs of column (b = r, f) -> exact integers (in place of
     // the tile), and the bra columns' magnitude keys: Ec + exponent of |S_0| +
@@ -506,7 +513,6 @@ __global__ void __launch_bounds__(kT64Threads, 1)
       }
       store_digits<NV>(sA, S::A_BYTES, tc_kmajor_offset(mc, hc * D + cc * NV, S::SBO), u, sg);
     }
-    const uint64_t tn = t + gstep;
     if (gtid == 0 && tn < ntiles) tc::mbar_arrive_expect_tx(&gp.full, S::TX_BYTES);  // the group's next tile
     tc::fence_proxy_async_smem();
     tc::fence_before_sync();
@@ -520,7 +526,7 @@ __global__ void __launch_bounds__(kT64Threads, 1)
     }
     pendm = 1;
     if (gtid < 128) gp.brmax[gtid] = 0;  // the next tile's magnitude keys
-    const uint64_t nbase = tn < ntiles ? tile_base_s(tn) : 0;
+    const uint64_t nbase = gp.nbase;
     if (tn < ntiles) {
       copy_tile(nbase);
       pendf = 1;
@@ -597,7 +603,8 @@ static cudaError_t launch_tc64_k(const LaunchArgs& a, cudaStream_t s) {
     configured = 1;
   }
   k_pass_tc64<K><<<a.grid, kT64Threads, t64_smem_bytes<K>(), s>>>(
-      static_cast<uint64_t*>(a.re), static_cast<uint64_t*>(a.im), static_cast<const TcDesc64<K>*>(a.desc), a.err);
+      static_cast<uint64_t*>(a.re), static_cast<uint64_t*>(a.im), static_cast<const TcDesc64<K>*>(a.desc), a.err,
+      a.half, a.herm);
   return cudaGetLastError();
 }
 

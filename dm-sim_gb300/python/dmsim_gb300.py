@@ -14,7 +14,7 @@ LIB_PATH = os.path.normpath(os.path.join(_HERE, "..", "lib", "libdmsim_gb300.so"
 
 OK, ERR_ARG, ERR_STATE, ERR_OOM, ERR_CUDA, ERR_TIMEOUT, ERR_UNSUPPORTED = range(7)
 (OPT_MODE, OPT_PRECISION, OPT_MAX_K, OPT_PLANNER, OPT_RECORD, OPT_SEED, OPT_GRAPH, OPT_VERBOSE, OPT_FUSED_ARITH,
- OPT_RENORM, OPT_PLAIN_ARITH, OPT_TENSOR, OPT_DIRECT1) = range(1, 14)
+ OPT_RENORM, OPT_PLAIN_ARITH, OPT_TENSOR, OPT_DIRECT1, OPT_HERMITIAN) = range(1, 15)
 AR_FP64, AR_FP32, AR_DF64 = 0, 1, 2
 BATCH_OPT_WAIT_LIMIT, BATCH_OPT_TEST_STALL, BATCH_OPT_WIDE_QUBITS = 100, 101, 102
 PASS_RECORD = 10  # doubles per pass record: K, class, nnz, max_lo_bit, min_hi_bit, n, ms, bytes, tensor, blocks

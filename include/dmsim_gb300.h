@@ -53,8 +53,11 @@ enum dmsim_option {
                                  FP64-width run, the 4-qubit passes of a complex64 run (BF16 x 3 split, FP32
                                  accumulation) and, in double-float runs, passes above a density rule [1];
                                  0 = never; 2 = every eligible pass */
-  DMSIM_OPT_DIRECT1 = 13      /* 1 = 1-qubit move/sign/phase/dense passes on the register kernel (no shared-memory
+  DMSIM_OPT_DIRECT1 = 13,     /* 1 = 1-qubit move/sign/phase/dense passes on the register kernel (no shared-memory
                                  tiles) [1], 0 = the tiled kernel */
+  DMSIM_OPT_HERMITIAN = 14    /* 1 = passes may compute one of every two Hermitian partners rho[r][c], rho[c][r] and
+                                 copy the other [1]; a rho written through dmsim_set_dm or the device pointers is
+                                 first checked, and runs in full when it is not Hermitian; 0 = every pass in full */
 };
 
 /* Gate ids: the order of enum OP, src/dmsim_nvgpu_omp.cuh:42-48 (ABI). */
