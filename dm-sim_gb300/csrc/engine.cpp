@@ -262,7 +262,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
 // What a pass takes, for the choice of half-range passes (plan_half): time
 // per entry as measured on GB300, tensor passes in whole rounds of the tiles
 // that run at once.
-HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, uint64_t ntiles) {
+HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, const PassSpec& spec, uint64_t ntiles) {
   HalfCost c;
   c.allowed = 0;
   c.fixed_us = 2.5;
@@ -282,7 +282,10 @@ HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, uint64_t ntiles) {
   if (p.cls == CLS_DENSE) fma = 2.0 * D * (p.real ? 2 : 4);
   else if (p.cls == CLS_SPARSE) fma = 2.0 * p.feat.nnz / D * (p.real ? 2 : 4);
   else if (p.cls == CLS_PHASE) fma = p.K > 1 ? 4.5 * p.feat.st_frac : 2;
-  else if (p.cls == CLS_SUPER) fma = 4.0 * D * D * 1.8;
+  else if (p.cls == CLS_SUPER) {
+    for (int i = 0; i < D * D * D * D; i++) fma += spec.U[i] == cplx(0, 0) ? 0 : spec.U[i].imag() == 0 ? 2 : 4;
+    fma /= D * D;
+  }
   c.slots = 1;
   c.tiles = 1000;  // no rounding: many small tiles
   c.tile_us = N * std::max(bw, fma * rate) * 1e-6 / c.tiles;
@@ -419,7 +422,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     }
     s->passes.push_back(pi);
     const PassHeader& hd = *reinterpret_cast<const PassHeader*>(blob.data() + offs[i]);
-    HalfCost hc = half_cost(s, pi, ntiles);
+    HalfCost hc = half_cost(s, pi, specs[i], ntiles);
     hc.allowed = half_allowed(hd, specs[i], (int)s->n, pi.direct1);
     costs.push_back(hc);
     std::array<int32_t, 10> gm = {hd.L, hd.mhi};

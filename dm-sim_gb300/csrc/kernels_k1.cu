@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   constexpr int CLS = base_class(CLS_);
   constexpr bool RE = real_class(CLS_);
   constexpr bool kMono = CLS == CLS_MOVE || CLS == CLS_SIGNED || CLS == CLS_PHASE;
+  constexpr bool kSuper = CLS == CLS_SUPER;
   const PassOp<1>& op = dp->op;
   // the operator, uniform over the grid (a few dozen bytes from L1)
   T ur[4], ui[4], vr[4], vi[4], fr[4], fi[4];
@@ -43,6 +44,27 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   src[1] = op.src[1];
   srcb[0] = op.srcb[0];
   srcb[1] = op.srcb[1];
+  // a channel's superoperator, and its nonzero terms: bit 4 o + j for output
+  // o = 2a + b and input j = 2c + e
+  __shared__ T s_sr[kSuper ? 16 : 1], s_si[kSuper ? 16 : 1];
+  __shared__ uint32_t s_nz, s_cplx;
+  uint32_t nz = 0, cplx = 0;
+  if constexpr (kSuper) {
+    if (threadIdx.x < 32) {
+      const int i = threadIdx.x & 15;
+      const double mr = op.sre[i], mi = op.sim[i];
+      s_sr[i] = coef<T>(mr);
+      s_si[i] = coef<T>(mi);
+      const uint32_t m = __ballot_sync(0xffffffffu, mr != 0.0 || mi != 0.0), mc = __ballot_sync(0xffffffffu, mi != 0.0);
+      if (threadIdx.x == 0) {
+        s_nz = m & 0xFFFFu;
+        s_cplx = mc & 0xFFFFu;
+      }
+    }
+    __syncthreads();
+    nz = s_nz;
+    cplx = s_cplx;
+  }
   // entry e = a + 2b: which change, which are read (unrolled comparisons,
   // so that the small arrays stay in registers)
   int sidx[4];
@@ -107,6 +129,27 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
           outi[e] = flip(r);
         }
       }
+    } else if constexpr (kSuper) {
+      // the terms in index order, the zero ones skipped (the same for every thread)
+#pragma unroll
+      for (int o = 0; o < 4; o++) {
+        T ar = 0, ai = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (!((nz >> (4 * o + j)) & 1)) continue;
+          const int x = (j >> 1) + 2 * (j & 1);
+          const T mr = s_sr[4 * o + j];
+          ar = madd(mr, xr[x], ar);
+          ai = madd(mr, xi[x], ai);
+          if ((cplx >> (4 * o + j)) & 1) {
+            const T mi = s_si[4 * o + j];
+            ar = madd(-mi, xi[x], ar);
+            ai = madd(mi, xr[x], ai);
+          }
+        }
+        outr[(o >> 1) + 2 * (o & 1)] = ar;
+        outi[(o >> 1) + 2 * (o & 1)] = ai;
+      }
     } else {
       // ket step: y[a][b] = sum_c U[a][c] x[c][b]
       T yr[4], yi[4];
@@ -169,13 +212,16 @@ cudaError_t launch1_t(const LaunchArgs& a, cudaStream_t s) {
     case CLS_SIGNED: return launch1<T, CLS_SIGNED>(a, s);
     case CLS_PHASE: return launch1<T, CLS_PHASE>(a, s);
     case CLS_DENSE: return a.real ? launch1<T, CLS_DENSE_REAL>(a, s) : launch1<T, CLS_DENSE>(a, s);
+    case CLS_SUPER: return launch1<T, CLS_SUPER>(a, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 }  // namespace
 
-bool direct1_class(int cls) { return cls == CLS_MOVE || cls == CLS_SIGNED || cls == CLS_PHASE || cls == CLS_DENSE; }
+bool direct1_class(int cls) {
+  return cls == CLS_MOVE || cls == CLS_SIGNED || cls == CLS_PHASE || cls == CLS_DENSE || cls == CLS_SUPER;
+}
 
 cudaError_t launch_pass1(const LaunchArgs& a, cudaStream_t s) {
   if (a.K != 1 || !direct1_class(a.cls)) return cudaErrorInvalidValue;

@@ -248,7 +248,11 @@ struct PassTables {
   int8_t src[D], srcb[D], nnz[D], nnzb[D];
   int8_t col[CLS == CLS_SPARSE ? D * D : 1], colb[CLS == CLS_SPARSE ? D * D : 1];
   int nnzmax, nnzbmax;
-  T ssr[CLS == CLS_SUPER && K <= 2 ? D * D * D * D : 1], ssi[CLS == CLS_SUPER && K <= 2 ? D * D * D * D : 1];
+  // SUPER: per output its nonzero inputs (index order), their number, whether any coefficient is complex
+  static constexpr int DD = CLS == CLS_SUPER && K <= 2 ? D * D : 1;
+  T ssr[DD * DD], ssi[DD * DD];
+  int soff[DD * DD];  // swizzled shared-memory offset of the input
+  int scnt[DD], scplx[DD];
 };
 
 template <typename T, int K, int CLS>
@@ -316,9 +320,22 @@ __device__ void load_tables(const PassDesc<K>* __restrict__ dp, PassTables<T, K,
     tb.rl[16 + tid] = coef<T>(dp->op.rlinb[tid]);
   }
   if constexpr (CLS == CLS_SUPER && K <= 2) {
-    for (int i = tid; i < D * D * D * D; i += blockDim.x) {
-      tb.ssr[i] = coef<T>(dp->op.sre[i]);
-      tb.ssi[i] = coef<T>(dp->op.sim[i]);
+    constexpr int DD = D * D;
+    if (tid < DD) {
+      int cnt = 0, cplx = 0;
+      for (int j = 0; j < DD; j++) {
+        const double mr = dp->op.sre[tid * DD + j], mi = dp->op.sim[tid * DD + j];
+        if (mr == 0.0 && mi == 0.0) continue;
+        int off = 0;
+        for (int i = 0; i < K; i++)
+          off |= (((j / D) >> i) & 1) << h.lket[i] | (((j % D) >> i) & 1) << h.lbra[i];
+        tb.ssr[tid * DD + cnt] = coef<T>(mr);
+        tb.ssi[tid * DD + cnt] = coef<T>(mi);
+        tb.soff[tid * DD + cnt++] = tile_sw<T>(off);
+        cplx |= mi != 0.0;
+      }
+      tb.scnt[tid] = cnt;
+      tb.scplx[tid] = cplx;
     }
   }
 }
@@ -438,33 +455,53 @@ __device__ void tile_body(T* __restrict__ re, T* __restrict__ im, const PassHead
   const int slf = tile_sw<T>(lf);
 
   if constexpr (CLS == CLS_SUPER && K <= 2) {
-    // ---- channel: each group's 4^K entries (a, b) <- S (4^K x 4^K), one thread per group
+    // ---- channel: each group's 4^K entries (a, b) <- S (4^K x 4^K), 2^K
+    // threads a group, 2^K outputs a thread, each the sum of its nonzero
+    // terms.  FP64's multiply-adds bound a dense S (64 an entry at K = 2, 12
+    // of 16 warps' worth of them for zeros in the named channels, whose rows
+    // hold 1 to 4 real terms: those are bound by memory).  A warp's threads
+    // share their outputs, so the term lists are broadcasts.  11 qubits, in
+    // 2-qubit depolarising: 970 us a pass with all 256 terms on one thread a
+    // group.
     constexpr int DD = D * D;
-    if (tid < G) {
-      int ls = 0;
-      for (int j = 0; j < g; j++) ls |= ((tid >> j) & 1) << h.freepos[j];
-      ls = tile_sw<T>(ls);
-      T xr[DD], xi[DD];
+    T yr[D], yi[D];
+    const bool has_out = tid < G * D;
+    const int part = tid >> g;
+    if (has_out) {
 #pragma unroll
-      for (int ab = 0; ab < DD; ab++) {
-        const int loc = ls ^ tb.lk[ab / D] ^ tb.lb[ab % D];
-        xr[ab] = sre[loc];
-        xi[ab] = sim[loc];
-      }
-#pragma unroll
-      for (int o = 0; o < DD; o++) {
+      for (int u = 0; u < D; u++) {
+        const int o = part * D + u;
         T ar = 0, ai = 0;
-#pragma unroll
-        for (int j = 0; j < DD; j++) {
-          const T mr = tb.ssr[o * DD + j], mi = tb.ssi[o * DD + j];
-          ar = madd(mr, xr[j], ar);
-          ar = madd(-mi, xi[j], ar);
-          ai = madd(mr, xi[j], ai);
-          ai = madd(mi, xr[j], ai);
+        const int cnt = tb.scnt[o];
+        if (tb.scplx[o]) {
+          for (int j = 0; j < cnt; j++) {
+            const T mr = tb.ssr[o * DD + j], mi = tb.ssi[o * DD + j];
+            const int loc = slf ^ tb.soff[o * DD + j];
+            const T xr = sre[loc], xi = sim[loc];
+            ar = madd(mr, xr, ar);
+            ar = madd(-mi, xi, ar);
+            ai = madd(mr, xi, ai);
+            ai = madd(mi, xr, ai);
+          }
+        } else {
+          for (int j = 0; j < cnt; j++) {
+            const T mr = tb.ssr[o * DD + j];
+            const int loc = slf ^ tb.soff[o * DD + j];
+            ar = madd(mr, sre[loc], ar);
+            ai = madd(mr, sim[loc], ai);
+          }
         }
-        const int loc = ls ^ tb.lk[o / D] ^ tb.lb[o % D];
-        sre[loc] = ar;
-        sim[loc] = ai;
+        yr[u] = ar;
+        yi[u] = ai;
+      }
+    }
+    __syncthreads();
+    if (has_out) {
+#pragma unroll
+      for (int u = 0; u < D; u++) {
+        const int loc = slf ^ tb.lk[part] ^ tb.lb[u];
+        sre[loc] = yr[u];
+        sim[loc] = yi[u];
       }
     }
     __syncthreads();
