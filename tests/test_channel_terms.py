@@ -32,7 +32,9 @@ def test_channel_terms(engine, kind, n, qubits, direct1):
     kraus = kraus_set(kind, len(qubits), rng)
     d = 1 << n
     a = (rng.standard_normal((d, d)) + 1j * rng.standard_normal((d, d))) / d
-    want = sum(embed(k, qubits, n) @ a @ embed(k, qubits, n).conj().T for k in kraus)
+    # a 2-qubit matrix's index is 2 bit(qubits[1]) + bit(qubits[0]) as the engine takes it
+    ops = [embed(k, qubits[::-1], n) for k in kraus]
+    want = sum(k @ a @ k.conj().T for k in ops)
     with engine.Simulation(n, mode="plain", direct1=direct1) as s:
         s.set_dm(a.T.real.reshape(-1), a.T.imag.reshape(-1))
         s.append_channel(qubits, kraus)
