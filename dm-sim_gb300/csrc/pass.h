@@ -166,11 +166,13 @@ DMG_HD constexpr uint32_t tc_kmajor_offset(uint32_t row, uint32_t k, uint32_t sb
 
 // ---- FP64-width tensor-core passes (K = 3, 4; FP64 state)
 // Every operand value is an integer on a power-of-two grid, split into 7
-// balanced base-256 digits (|digit| <= 128, exact in BF16): 55 significant
+// balanced base-256 digits (|digit| <= 128, exact in FP16): 55 significant
 // bits for the largest value of each column of the state, 56 for each row
 // of the operator.  Slice pairs of orders i + j = 0..7 accumulate exactly in
 // FP32 (every partial sum is an integer below 2^22), the orders are combined
-// in 64-bit integer arithmetic and rounded once to FP64.
+// in 64-bit integer arithmetic and rounded once to FP64.  The state's digits
+// are stored as digit + 128 times 2^-24 (a byte is that FP16 subnormal as it
+// is); the sums start 128 times the operator's digits lower.
 constexpr int kTc64Slices = 7;
 constexpr int kTc64Orders = 8;
 
@@ -182,8 +184,12 @@ struct TcDesc64 {
   // sum_j digit_j 256^(6-j); rows n and n + D (the real and imaginary parts
   // of output n) hold the same magnitudes and share the exponent.
   int32_t ew[2][D];
-  // digits j = 0..6 of W (0) and V (1): BF16 bits, K-major core-matrix layout
+  // digits j = 0..6 of W (0) and V (1): FP16 bits, K-major core-matrix layout
   alignas(16) uint16_t sl[2][kTc64Slices][R * R];
+  // the order sums' starting values 0.75 - 128 2^-24 C, C = sum over the slice
+  // pairs of order o and over k of w_j[n][k]: row o R + n is the FP16 numbers
+  // 0.75, -c1 2^-9, -c0 2^-17 and five zeros, C = 256 c1 + c0, |c0| <= 128
+  alignas(16) uint16_t start[2][kTc64Orders * R * 8];
 };
 
 template <int K>

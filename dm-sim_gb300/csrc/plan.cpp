@@ -658,6 +658,29 @@ void tc64_digits(int64_t t, int d[7]) {
   d[0] = (int)(u >> 48) - 128;
 }
 
+// FP16 bits of an integer |i| < 2048 times 2^e, exact in FP16 (a multiple of 2^-24).
+static uint16_t f16_scaled(int i, int e) {
+  if (i == 0) return 0;
+  const uint16_t sign = i < 0 ? 0x8000 : 0;
+  int m = i < 0 ? -i : i, ex = e;  // value m 2^ex; bring m to 11 bits
+  while (m < 1024 && ex > -24) {
+    m <<= 1;
+    ex--;
+  }
+  if (m < 1024) return (uint16_t)(sign | m);                // subnormal: ex = -24
+  return (uint16_t)(sign | ((ex + 25) << 10) | (m - 1024));  // 1.f 2^(ex + 10), bias 15
+}
+
+namespace {
+struct F16Digits {  // the digits' FP16 bits
+  uint16_t bits[257];
+  F16Digits() {
+    for (int i = -128; i <= 128; i++) bits[i + 128] = f16_scaled(i, 0);
+  }
+  uint16_t operator()(int i) const { return bits[i + 128]; }
+};
+}  // namespace
+
 // The FP64-width descriptor: the geometry of the double-float tensor pass and
 // the operator's rows as 56-bit integers times a power of two, in digits.
 template <int K>
@@ -676,7 +699,9 @@ uint64_t build_tc64_k(const PassSpec& p, int n, TcDesc64<K>* d, PassFeatures* fe
     nst += (h.stmask[r >> 5] >> (r & 31)) & 1;
   }
   if (feat) feat->ld_frac = 1.0;
-  for (int side = 0; side < 2 && slices; side++) {
+  if (!slices) return (uint64_t)(nst + nruns) * (1ull << h.L) * h.ntiles;
+  static const F16Digits f16;
+  for (int side = 0; side < 2; side++) {
     const cplx* M = side ? p.V : p.U;
     for (int a = 0; a < D; a++) {
       // rows a ([Ur, -Ui]) and a + D ([Ui, Ur]) hold the same magnitudes
@@ -685,22 +710,34 @@ uint64_t build_tc64_k(const PassSpec& p, int n, TcDesc64<K>* d, PassFeatures* fe
       int e = 0;
       if (mx > 0) std::frexp(mx, &e);  // every |entry| < 2^e
       d->ew[side][a] = mx > 0 ? e - 55 : 0;
-      for (int half = 0; half < 2; half++) {
-        const int row = a + half * D;
-        for (int k = 0; k < R; k++) {
-          const cplx m = M[a * D + (k % D)];
-          const double w = half == 0 ? (k < D ? m.real() : -m.imag()) : (k < D ? m.imag() : m.real());
-          const int64_t t = mx > 0 ? (int64_t)std::nearbyint(std::ldexp(w, 55 - e)) : 0;  // |t| <= 2^55
-          int dg[7];
-          tc64_digits(t, dg);
-          for (int j = 0; j < kTc64Slices; j++) {
-            const float tf = (float)dg[j];  // |digit| <= 128: exact in BF16
-            uint32_t bits;
-            std::memcpy(&bits, &tf, 4);
-            d->sl[side][j][tc_kmajor_offset(row, k, 16 * R) / 2] = (uint16_t)(bits >> 16);
-          }
+      const double scale = std::ldexp(1.0, 55 - e);
+      int rowsum[2][kTc64Slices] = {{0}};
+      for (int k = 0; k < D; k++) {
+        const cplx m = M[a * D + k];
+        int dr[7], di[7];  // |t| <= 2^55; the digits of -t are t's negated
+        tc64_digits(mx > 0 ? (int64_t)std::nearbyint(m.real() * scale) : 0, dr);
+        tc64_digits(mx > 0 ? (int64_t)std::nearbyint(m.imag() * scale) : 0, di);
+        const uint32_t o00 = tc_kmajor_offset(a, k, 16 * R) / 2, o01 = tc_kmajor_offset(a, k + D, 16 * R) / 2,
+                       o10 = tc_kmajor_offset(a + D, k, 16 * R) / 2, o11 = tc_kmajor_offset(a + D, k + D, 16 * R) / 2;
+        for (int j = 0; j < kTc64Slices; j++) {
+          uint16_t* sl = d->sl[side][j];
+          sl[o00] = sl[o11] = f16(dr[j]);
+          sl[o10] = f16(di[j]);
+          sl[o01] = f16(-di[j]);
+          rowsum[0][j] += dr[j] - di[j];
+          rowsum[1][j] += dr[j] + di[j];
         }
       }
+      for (int half = 0; half < 2; half++)
+        for (int o = 0; o < kTc64Orders; o++) {
+          int C = 0;  // over the pairs (o - j, j), both below kTc64Slices
+          for (int j = std::max(0, o - kTc64Slices + 1); j <= std::min(o, kTc64Slices - 1); j++) C += rowsum[half][j];
+          const int c1 = (C + 128) >> 8, c0 = C - 256 * c1;
+          uint16_t* st = d->start[side] + ((size_t)o * R + a + half * D) * 8;
+          st[0] = f16_scaled(3, -2);
+          st[1] = f16_scaled(-c1, -9);
+          st[2] = f16_scaled(-c0, -17);
+        }
     }
   }
   const uint64_t runlen = 1ull << h.L;

@@ -43,6 +43,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
+// The same with A and B FP16 (bits [7,10) and [10,13) = 0).
+__host__ __device__ constexpr uint32_t idesc_f16_f32(uint32_t M, uint32_t N) {
+  return (1u << 4) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
 // ---- tensor memory (one warp, all 32 lanes)
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot_smem)),
@@ -127,8 +132,8 @@ __device__ __forceinline__ bool named_bar_or(int id, bool p) {
   return r != 0;
 }
 
-// ---- MMA: D[tmem] (+)= A[smem] * B[smem]^T, one thread issues
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// ---- MMA: D[tmem] (+)= A[smem] * B[smem]^T, one thread issues; kind::f16 (the descriptor says FP16 or BF16)
+__device__ __forceinline__ void mma_f16kind(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -154,6 +159,16 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
                    smem_u32(smem_dst)),
                "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
+}
+
+// ---- 16-byte asynchronous copies global -> shared (cp.async), both addresses
+// 16-byte aligned; cp_async_arrive arrives on an mbarrier once all of this
+// thread's earlier ones have landed
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // ---- TMEM -> registers: this warp's 32 lanes, 4 / 8 / 16 consecutive columns

@@ -224,7 +224,7 @@ __device__ bool tc_step(T* __restrict__ sre, T* __restrict__ sim, unsigned char*
       for (int kk = 0; kk < R / 16; kk++) {
         const uint64_t ad = tc::smem_desc(a0 + i * SH::A_BYTES + kk * 256, tc::kLbo, SH::SBO);
         const uint64_t bd = tc::smem_desc(b0 + j0 * SH::B_BYTES + kk * 256, tc::kLbo, SH::SBO);
-        tc::mma_bf16(tmem + (i + j0) * R, ad, bd, tc::idesc_bf16_f32(128, nb * R), (overwrite && kk == 0) ? 0u : 1u);
+        tc::mma_f16kind(tmem + (i + j0) * R, ad, bd, tc::idesc_bf16_f32(128, nb * R), (overwrite && kk == 0) ? 0u : 1u);
       }
     };
     constexpr int O = SH::ORDERS;

@@ -159,7 +159,7 @@ __device__ __forceinline__ void issue_step32(const unsigned char* sA, const unsi
     for (int kk = 0; kk < R / 16; kk++) {
       const uint64_t ad = tc::smem_desc(a0 + kPairs[q][0] * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
       const uint64_t bd = tc::smem_desc(b0 + kPairs[q][1] * S::B_BYTES + kk * 256, tc::kLbo, S::SBO);
-      tc::mma_bf16(dset, ad, bd, tc::idesc_bf16_f32(128, R), (q == 0 && kk == 0) ? 0u : 1u);
+      tc::mma_f16kind(dset, ad, bd, tc::idesc_bf16_f32(128, R), (q == 0 && kk == 0) ? 0u : 1u);
     }
   }
 }
