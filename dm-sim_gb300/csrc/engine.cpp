@@ -194,6 +194,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.real = p.real;
     a.err = s->d_err;
     a.direct1 = p.direct1;
+    a.mono = p.mono;
     a.q0 = p.q0;
     a.n = (int)s->n;
     a.half = p.half ? reinterpret_cast<const HalfMap*>(static_cast<const char*>(s->d_desc) + p.half_off) : nullptr;
@@ -413,6 +414,11 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     const int bps = pi.tc ? tc_blocks_per_sm(pi.K, arith) : pass_blocks_per_sm(pi.K, pi.cls, arith);
     const uint64_t cap = (uint64_t)s->sms * (uint64_t)bps;
     pi.grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ntiles, cap));
+    if (!pi.tc)
+      if (const unsigned g = mono_grid(pi.K, pi.cls, tile, ntiles, s->sms)) {
+        pi.mono = true;
+        pi.grid = g;
+      }
     // 1-qubit passes (n >= 2): one register-resident group of 4 entries per thread
     pi.q0 = specs[i].q[0];
     pi.direct1 = s->direct1 && !pi.tc && pi.K == 1 && s->n >= 2 && direct1_class(pi.cls);

@@ -23,6 +23,7 @@ struct PassInfo {
   bool tc;              // runs on the tensor cores (tensor.cu)
   bool real;            // real operator (kernels_real.cu for K <= 2)
   bool direct1;         // 1-qubit pass on the register kernel (kernels_k1.cu)
+  bool mono;            // monomial pass on the pipelined kernel (kernels_mono.cu)
   int q0;               // first target qubit
   uint32_t half;        // half-range pass: its qubit set S (0: the whole state)
   uint32_t stale;       // the set under which the state is up to date before the pass: a mirror pass goes first

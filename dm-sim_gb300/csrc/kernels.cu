@@ -78,6 +78,7 @@ cudaError_t launch_pass(const LaunchArgs& a, cudaStream_t s) {
     return launch_pass_tc(a, s);
   }
   if (a.direct1) return launch_pass1(a, s);
+  if (a.mono) return launch_mono(a, s);
   if (a.arith == AR_DF64) return launch_t<df64>(a, s);
   return a.fp32 ? launch_t<float>(a, s) : launch_t<double>(a, s);
 }

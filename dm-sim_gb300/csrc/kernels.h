@@ -24,6 +24,7 @@ struct LaunchArgs {
                        // for an FP64 state, a TcDesc64<K>
   int* err;            // device flag set to 1 when a bounded wait of a tensor pass runs out
   bool direct1;        // 1-qubit pass run by the register kernel (kernels_k1.cu)
+  bool mono;           // monomial pass on the pipelined kernel (kernels_mono.cu)
   int q0, n;           // its qubit and the state's qubit count
   const HalfMap* half; // device map of a half-range pass (pass.h), else null
   const int* herm;     // device flag: half-range passes run on the half range (the state is Hermitian)
@@ -36,6 +37,10 @@ int pass_blocks_per_sm(int K, int cls, int arith);
 // 1-qubit MOVE / SIGNED / PHASE / DENSE passes without shared memory (kernels_k1.cu).
 bool direct1_class(int cls);
 cudaError_t launch_pass1(const LaunchArgs& a, cudaStream_t s);
+// Monomial passes of 2 to 4 qubits on states of many tiles (kernels_mono.cu): its
+// grid, 0 for a pass that it does not take, and the launch.
+unsigned mono_grid(int K, int cls, int tile_entries, uint64_t ntiles, int sms);
+cudaError_t launch_mono(const LaunchArgs& a, cudaStream_t s);
 // Real-operator instances of the 1- and 2-qubit DENSE/SPARSE kernels (kernels_real.cu).
 cudaError_t launch_pass_real(const LaunchArgs& a, cudaStream_t s);
 // Tensor-core passes (tensor.cu): launch, and resident blocks per SM.
