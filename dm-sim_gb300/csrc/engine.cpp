@@ -192,6 +192,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.tile_entries = p.tile_entries;
     a.tc = p.tc;
     a.real = p.real;
+    a.hadamard = p.hadamard;
     a.err = s->d_err;
     a.direct1 = p.direct1;
     a.mono = p.mono;
@@ -280,7 +281,7 @@ HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, const PassSpec& spec, 
   const double rate = s->arith == AR_FP64 ? 2.0 : 0.6;  // per multiply-add
   const int D = 1 << p.K;
   double fma = 0;
-  if (p.cls == CLS_DENSE) fma = 2.0 * D * (p.real ? 2 : 4);
+  if (p.cls == CLS_DENSE) fma = p.hadamard && p.direct1 && s->arith == AR_FP64 ? 4 : 2.0 * D * (p.real ? 2 : 4);
   else if (p.cls == CLS_SPARSE) fma = 2.0 * p.feat.nnz / D * (p.real ? 2 : 4);
   else if (p.cls == CLS_PHASE) fma = p.K > 1 ? 4.5 * p.feat.st_frac : 2;
   else if (p.cls == CLS_SUPER) {
@@ -404,6 +405,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
               : build_desc(specs[i], (int)s->n, blob.data() + offs[i], &pi.feat, &ntiles, &tile);
     pi.feat.tc = pi.tc ? 1 : 0;
     pi.real = !pi.tc && pi.feat.real;
+    pi.hadamard = !pi.tc && pi.feat.hadamard;
     pi.K = specs[i].K;
     pi.cls = specs[i].cls;
     pi.desc_off = offs[i];

@@ -21,6 +21,7 @@ struct PassInfo {
   double bytes;         // algorithmic bytes moved (reads + writes)
   int nbasic;
   bool tc;              // runs on the tensor cores (tensor.cu)
+  bool hadamard;        // kPassHadamard pass (pass.h)
   bool real;            // real operator (kernels_real.cu for K <= 2)
   bool direct1;         // 1-qubit pass on the register kernel (kernels_k1.cu)
   bool mono;            // monomial pass on the pipelined kernel (kernels_mono.cu)

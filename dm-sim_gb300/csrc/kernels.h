@@ -19,6 +19,7 @@ struct LaunchArgs {
   int arith;           // Arith
   unsigned grid;       // blocks
   int tile_entries;    // G * 4^K
+  bool hadamard;       // kPassHadamard pass (pass.h)
   bool real;           // DENSE/SPARSE pass whose U and V are real (pass.h kPassRealOperator)
   bool tc;             // tensor-core pass, K = 3, 4: desc is a TcDesc<K> (double-float or FP32 state) or,
                        // for an FP64 state, a TcDesc64<K>

@@ -10,12 +10,32 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "kernels.h"
 #include "pass_device.cuh"
 
 namespace dmg {
 
 namespace {
+
+// x / 2: one off the exponent field, on the ALU, where that is exact; zeros are
+// themselves.
+__device__ __forceinline__ double half_of(double x) {
+  const int h = __double2hiint(x), l = __double2loint(x);
+  const uint32_t e = (uint32_t)h & 0x7FF00000u;
+  if (e == 0x00100000u || e == 0x7FF00000u || (e == 0 && ((h << 1) | l))) return 0.5 * x;
+  return __hiloint2double(h - (e ? 0x00100000 : 0), l);
+}
+// -x if n (32-bit integer work: a select of doubles takes the FP64 pipe)
+__device__ __forceinline__ double xor_sign(double x, bool n) {
+  return __hiloint2double(__double2hiint(x) ^ (n ? (int)0x80000000 : 0), __double2loint(x));
+}
+__device__ __forceinline__ float xor_sign(float x, bool n) { return n ? -x : x; }
+__device__ __forceinline__ df64 xor_sign(df64 x, bool n) { return n ? -x : x; }
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ df64 half_of(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
+__device__ __forceinline__ df64 operator-(df64 a, df64 b) { return a + -b; }
 
 template <typename T, int CLS_>
 __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict__ im,
@@ -25,6 +45,7 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   constexpr bool RE = real_class(CLS_);
   constexpr bool kMono = CLS == CLS_MOVE || CLS == CLS_SIGNED || CLS == CLS_PHASE;
   constexpr bool kSuper = CLS == CLS_SUPER;
+  constexpr bool kHad = CLS_ == CLS_HADAMARD;
   const PassOp<1>& op = dp->op;
   // the operator, uniform over the grid (a few dozen bytes from L1)
   T ur[4], ui[4], vr[4], vi[4], fr[4], fi[4];
@@ -82,6 +103,7 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
     need[e] = nd;
   }
 
+  const bool hswap = kHad && op.ure[0] * op.ure[1] < 0, hneg = kHad && op.ure[0] * op.ure[2] < 0;
   const HalfMap* hm = half && *herm ? half : nullptr;  // the half range of the groups, if any
   const uint64_t ngroups = hm ? hm->count : 1ull << (2 * n - 2);
   const uint64_t mq = 1ull << q, mb = 1ull << (q + n);
@@ -128,6 +150,40 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
           outr[e] = m;
           outi[e] = flip(r);
         }
+      }
+    } else if constexpr (kHad) {
+      // sqrt(1/2) (1 1; 1 -1) on either side: sums and differences, a half of
+      // them exactly -- four FP64 additions an entry instead of eight
+      // multiply-adds, and no rounded sqrt(1/2).  Row a of U is rs_a (1, p_a)
+      // sqrt(1/2), p_0 = -p_1: out[a][b] = rs_a rs_b z[p_a < 0][p_b < 0], by the
+      // place it is stored at.  13 qubits, half range: 501 -> 300 us a pass (the
+      // FP64 pipe alone 223, HBM 167); with the outputs chosen by value, selects
+      // of doubles that run on the FP64 pipe, it took 567.
+      T z[2][4];  // real, imaginary parts; index i + 2 j
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const T* x = c ? xi : xr;
+        const T s0 = x[0] + x[1], d0 = x[0] - x[1], s1 = x[2] + x[3], d1 = x[2] - x[3];
+        z[c][0] = half_of(s0 + s1);
+        z[c][1] = half_of(d0 + d1);
+        z[c][2] = half_of(s0 - s1);
+        z[c][3] = half_of(d0 - d1);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        outr[e] = z[0][e];
+        outi[e] = z[1][e];
+        if (e == 1 || e == 2) {
+          outr[e] = xor_sign(outr[e], hneg);
+          outi[e] = xor_sign(outi[e], hneg);
+        }
+      }
+      if (hswap) {
+        const uint64_t a = idx[0], b = idx[1];
+        idx[0] = idx[3];
+        idx[1] = idx[2];
+        idx[2] = b;
+        idx[3] = a;
       }
     } else if constexpr (kSuper) {
       // the terms in index order, the zero ones skipped (the same for every thread)
@@ -211,7 +267,9 @@ cudaError_t launch1_t(const LaunchArgs& a, cudaStream_t s) {
     case CLS_MOVE: return launch1<T, CLS_MOVE>(a, s);
     case CLS_SIGNED: return launch1<T, CLS_SIGNED>(a, s);
     case CLS_PHASE: return launch1<T, CLS_PHASE>(a, s);
-    case CLS_DENSE: return a.real ? launch1<T, CLS_DENSE_REAL>(a, s) : launch1<T, CLS_DENSE>(a, s);
+    case CLS_DENSE:
+      if (a.hadamard && std::is_same<T, double>::value) return launch1<T, CLS_HADAMARD>(a, s);
+      return a.real ? launch1<T, CLS_DENSE_REAL>(a, s) : launch1<T, CLS_DENSE>(a, s);
     case CLS_SUPER: return launch1<T, CLS_SUPER>(a, s);
     default: return cudaErrorInvalidValue;
   }

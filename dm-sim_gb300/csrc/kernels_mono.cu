@@ -60,6 +60,20 @@ struct alignas(16) Chunk {
   T v[16 / sizeof(T)];
 };
 
+// c ? a : b, its sign flipped if neg.  Integer words: a select of doubles
+// takes the FP64 pipe.
+__device__ __forceinline__ double pick(bool c, double a, double b, bool neg) {
+  const int h = c ? __double2hiint(a) : __double2hiint(b), l = c ? __double2loint(a) : __double2loint(b);
+  return __hiloint2double(h ^ (neg ? (int)0x80000000 : 0), l);
+}
+__device__ __forceinline__ float pick(bool c, float a, float b, bool neg) {
+  const float x = c ? a : b;
+  return neg ? flip(x) : x;
+}
+__device__ __forceinline__ df64 pick(bool c, df64 a, df64 b, bool neg) {
+  return df64(pick(c, a.hi, b.hi, neg), pick(c, a.lo, b.lo, neg));
+}
+
 template <typename T, int K, int CLS>
 __global__ void __launch_bounds__(Mono<T, K>::NT, K <= 3 ? 2 : 1)
     k_mono(T* __restrict__ re, T* __restrict__ im, const PassDesc<K>* __restrict__ dp,
@@ -140,16 +154,17 @@ __global__ void __launch_bounds__(Mono<T, K>::NT, K <= 3 ? 2 : 1)
       for (int u = 0; u < V; u++) {
         const T vr = sre[src[c][u]], vi = sim[src[c][u]];
         const uint32_t fk = CLS == CLS_MOVE ? (uint32_t)FK_ONE : (kinds >> (3 * (c * V + u))) & 7u;
-        T r = vr, m = vi;
         if (CLS == CLS_PHASE && fk == FK_GEN) {
-          r = madd(fr[c][u], vr, -fi[c][u] * vi);
-          m = madd(fr[c][u], vi, fi[c][u] * vr);
-        } else if (CLS != CLS_MOVE && fk != FK_ONE) {
-          r = fk == FK_NEG ? flip(vr) : fk == FK_PI ? flip(vi) : vi;  // -x, i x = -vi + i vr, -i x = vi - i vr
-          m = fk == FK_NEG ? flip(vi) : fk == FK_PI ? vr : flip(vr);
+          wr.v[u] = madd(fr[c][u], vr, -fi[c][u] * vi);
+          wi.v[u] = madd(fr[c][u], vi, fi[c][u] * vr);
+        } else if (CLS == CLS_MOVE || (CLS == CLS_PHASE && fk == FK_ONE)) {
+          wr.v[u] = vr;
+          wi.v[u] = vi;
+        } else {  // -x, i x = -vi + i vr, -i x = vi - i vr
+          const bool swap = fk == FK_PI || fk == FK_NI;
+          wr.v[u] = pick(swap, vi, vr, fk == FK_NEG || fk == FK_PI);
+          wi.v[u] = pick(swap, vr, vi, fk == FK_NEG || fk == FK_NI);
         }
-        wr.v[u] = r;
-        wi.v[u] = m;
       }
       __stcg(reinterpret_cast<float4*>(re + base + goff[c]), *reinterpret_cast<const float4*>(&wr));
       __stcg(reinterpret_cast<float4*>(im + base + goff[c]), *reinterpret_cast<const float4*>(&wi));

@@ -46,9 +46,12 @@ enum PassClass : int32_t {
 constexpr int kClsRealOffset = 16;
 constexpr int CLS_DENSE_REAL = kClsRealOffset + CLS_DENSE;
 constexpr int CLS_SPARSE_REAL = kClsRealOffset + CLS_SPARSE;
-DMG_HD constexpr int base_class(int c) { return c >= kClsRealOffset ? c - kClsRealOffset : c; }
+DMG_HD constexpr int base_class(int c) { return c % kClsRealOffset; }
 DMG_HD constexpr bool real_class(int c) { return c >= kClsRealOffset; }
 constexpr int32_t kPassRealOperator = 1;  // PassHeader::flags bit
+constexpr int32_t kPassHadamard = 2;      // flags bit: 1 qubit, V = conj(U), every entry of U is +-sqrt(1/2)
+// Instance of the 1-qubit register kernel for kPassHadamard passes on an FP64 state.
+constexpr int CLS_HADAMARD = 2 * kClsRealOffset + 3;
 
 // Factor kinds of a monomial superoperator entry f[a][b].
 enum FactorKind : int8_t { FK_ONE = 0, FK_NEG = 1, FK_PI = 2, FK_NI = 3, FK_GEN = 4 };
@@ -58,7 +61,7 @@ struct PassHeader {
   int32_t L;         // low run bits
   int32_t mhi;       // number of target bits >= L
   int32_t g;         // log2 of groups per tile
-  int32_t flags;     // kPassRealOperator: U and V are real
+  int32_t flags;     // kPassRealOperator: U and V are real; kPassHadamard
   uint64_t ntiles;   // tiles in the state
   int32_t hipos[8];  // global positions of the high target bits, ascending
   int32_t lket[4];   // local bit position of ket target i (qubit q_i)

@@ -441,6 +441,16 @@ uint64_t build_k(const PassSpec& p, int n, PassDesc<K>* d, PassFeatures* feat, u
     real = real && op.uim[i] == 0.0 && op.vim[i] == 0.0;
   }
   if (real) h.flags |= kPassRealOperator;
+  // H and its like: real, unitary (an odd number of minus signs), magnitudes within 2 ulp of sqrt(1/2)
+  if (K == 1 && real && !p.ket_only) {
+    bool had = true;
+    int minus = 0;
+    for (int i = 0; i < 4; i++) {
+      had = had && std::fabs(std::fabs(op.ure[i]) - std::sqrt(0.5)) <= 2.3e-16;
+      minus += op.ure[i] < 0;
+    }
+    if (had && (minus & 1)) h.flags |= kPassHadamard;
+  }
   std::memcpy(op.rlin, p.rl, sizeof op.rlin);
   std::memcpy(op.rlinb, p.rlb, sizeof op.rlinb);
   if (p.cls == CLS_SUPER && K <= 2) {
@@ -553,6 +563,7 @@ uint64_t build_k(const PassSpec& p, int n, PassDesc<K>* d, PassFeatures* feat, u
     feat->cls = p.cls;
     feat->nnz = p.nnz;
     feat->real = real ? 1 : 0;
+    feat->hadamard = (h.flags & kPassHadamard) != 0;
     feat->n = n;
     int lo = -1, hmin = nb;
     for (int x : P) {
