@@ -431,7 +431,10 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     s->passes.push_back(pi);
     const PassHeader& hd = *reinterpret_cast<const PassHeader*>(blob.data() + offs[i]);
     HalfCost hc = half_cost(s, pi, specs[i], ntiles);
-    hc.allowed = half_allowed(hd, specs[i], (int)s->n, pi.direct1);
+    // tiled monomial passes (states of few tiles) have no half-range instance
+    const bool tiled_mono = !pi.tc && !pi.direct1 && !pi.mono && pi.K > 1 &&
+                            (pi.cls == CLS_MOVE || pi.cls == CLS_SIGNED || pi.cls == CLS_PHASE);
+    hc.allowed = tiled_mono ? 0 : half_allowed(hd, specs[i], (int)s->n, pi.direct1);
     costs.push_back(hc);
     std::array<int32_t, 10> gm = {hd.L, hd.mhi};
     for (int j = 0; j < hd.mhi; j++) gm[2 + j] = hd.hipos[j];
@@ -461,7 +464,10 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
   }
   // complex64 runs stay whole: their renormalisation averages the two
   // partners' FP32 rounding errors, which a copied partner would not have
-  if (s->hermitian && s->keeps_herm && !s->fp32 && s->n >= 6) total = plan_half_ranges(s, costs, geo, blob, total);
+  // states below 10 qubits (16 MB) run whole too: their passes are launch and
+  // latency, a half of them no shorter, and the mirrors come on top (9 qubits,
+  // 100 layered gates double-float 204 us whole, 253 us half; 10 qubits 376, 330)
+  if (s->hermitian && s->keeps_herm && !s->fp32 && s->n >= 10) total = plan_half_ranges(s, costs, geo, blob, total);
   if (total > 0) {
     DM_CUDA(cudaMalloc(&s->d_desc, total));
     DM_CUDA(cudaMemcpyAsync(s->d_desc, blob.data(), total, cudaMemcpyHostToDevice, s->stream));

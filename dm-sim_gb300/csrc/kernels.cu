@@ -88,8 +88,8 @@ static int occ_one() {
   constexpr int D = 1 << K;
   int nb = 0;
   const size_t smem = pass_smem_bytes<T, K, CLS>(kThreads * D);
-  if (configure_pass<T, K, CLS>() != cudaSuccess) return 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pass<T, K, CLS>, kThreads, smem) != cudaSuccess) return 1;
+  if (configure_pass<T, K, CLS, false>() != cudaSuccess) return 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pass<T, K, CLS, false>, kThreads, smem) != cudaSuccess) return 1;
   return nb > 0 ? nb : 1;
 }
 

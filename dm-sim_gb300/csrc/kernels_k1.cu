@@ -37,7 +37,7 @@ __device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
 __device__ __forceinline__ df64 half_of(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
 __device__ __forceinline__ df64 operator-(df64 a, df64 b) { return a + -b; }
 
-template <typename T, int CLS_>
+template <typename T, int CLS_, bool HALF>
 __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict__ im,
                                                const PassDesc<1>* __restrict__ dp, int q, int n,
                                                const HalfMap* __restrict__ half, const int* __restrict__ herm) {
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   }
 
   const bool hswap = kHad && op.ure[0] * op.ure[1] < 0, hneg = kHad && op.ure[0] * op.ure[2] < 0;
-  const HalfMap* hm = half && *herm ? half : nullptr;  // the half range of the groups, if any
+  const HalfMap* hm = HALF && *herm ? half : nullptr;  // the half range of the groups, if any
   const uint64_t ngroups = hm ? hm->count : 1ull << (2 * n - 2);
   const uint64_t mq = 1ull << q, mb = 1ull << (q + n);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -256,8 +256,15 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
 
 template <typename T, int CLS_>
 cudaError_t launch1(const LaunchArgs& a, cudaStream_t s) {
-  k_pass1<T, CLS_><<<a.grid, 256, 0, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                          static_cast<const PassDesc<1>*>(a.desc), a.q0, a.n, a.half, a.herm);
+  // two instances, as for the tiled kernel (pass_kernel.cuh)
+  auto* k = k_pass1<T, CLS_, false>;
+  if constexpr (!std::is_same<T, float>::value) {
+    if (a.half) k = k_pass1<T, CLS_, true>;
+  } else if (a.half) {
+    return cudaErrorInvalidValue;
+  }
+  k<<<a.grid, 256, 0, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im), static_cast<const PassDesc<1>*>(a.desc), a.q0,
+                           a.n, a.half, a.herm);
   return cudaGetLastError();
 }
 

@@ -12,16 +12,18 @@
 
 namespace dmg {
 
-// One pass over the whole state: the block stages the pass's tables once,
-// then grid-strides over the tiles.
-template <typename T, int K, int CLS>
+// One pass over the whole state or (HALF, pass.h) half of it: the block stages
+// the pass's tables once, then grid-strides over the tiles.  Two instances: with
+// the half range's tile numbering in it, a pass of a state that fits a few blocks
+// took 2 to 3 % longer (5 to 9 qubits, launch and latency).
+template <typename T, int K, int CLS, bool HALF>
 __global__ void __launch_bounds__(kThreads) k_pass(T* __restrict__ re, T* __restrict__ im,
                                                    const PassDesc<K>* __restrict__ dp,
                                                    const HalfMap* __restrict__ half, const int* __restrict__ herm) {
   constexpr int D = 1 << K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const PassHeader& h = dp->h;
-  const HalfMap* hm = half && *herm ? half : nullptr;
+  const HalfMap* hm = HALF && *herm ? half : nullptr;
   const uint64_t ntiles = hm ? hm->count : h.ntiles;
   const int tile = (1 << h.g) * D * D;
   T* sre = reinterpret_cast<T*>(smem_raw);
@@ -59,28 +61,42 @@ __global__ void __launch_bounds__(kThreads) k_pass(T* __restrict__ re, T* __rest
 // Dynamic shared memory for the largest tile, and the largest shared-memory
 // carveout so that the resident-block count the occupancy query reports is
 // the one the launches get.
-template <typename T, int K, int CLS>
+template <typename T, int K, int CLS, bool HALF>
 inline cudaError_t configure_pass() {
   constexpr int D = 1 << K;
-  cudaError_t e = cudaFuncSetAttribute(k_pass<T, K, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_pass<T, K, CLS, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)pass_smem_bytes<T, K, CLS>(kThreads * D));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_pass<T, K, CLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(k_pass<T, K, CLS, HALF>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
   return e;
 }
 
+// Whether a class has a half-range instance: complex64 passes run whole, and so
+// do the monomial ones of 2 qubits and more, but on the pipelined kernel.
 template <typename T, int K, int CLS>
+constexpr bool half_instance() {
+  constexpr int C = base_class(CLS);
+  if (std::is_same<T, float>::value || C == CLS_RLIN) return false;
+  return K == 1 || C == CLS_DENSE || C == CLS_SPARSE || C == CLS_SUPER;
+}
+
+template <typename T, int K, int CLS, bool HALF = false>
 inline cudaError_t launch_one(const LaunchArgs& a, cudaStream_t s) {
-  constexpr int D = 1 << K;
+  if constexpr (!HALF) {
+    if (a.half) {
+      if constexpr (half_instance<T, K, CLS>()) return launch_one<T, K, CLS, true>(a, s);
+      else return cudaErrorInvalidValue;
+    }
+  }
   const size_t smem = pass_smem_bytes<T, K, CLS>(a.tile_entries);
   static int configured = 0;  // per instance; attribute set once per process
   if (!configured) {
-    cudaError_t e = configure_pass<T, K, CLS>();
+    cudaError_t e = configure_pass<T, K, CLS, HALF>();
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_pass<T, K, CLS><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
+  k_pass<T, K, CLS, HALF><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
                                                    static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
   return cudaGetLastError();
 }

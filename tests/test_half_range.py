@@ -82,3 +82,24 @@ def test_half_sizes(engine, n):
             out.append(s.get_dm())
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arith", ["fp64", "df64"])
+def test_half_tiled_one_qubit_passes(engine, arith):
+    """The tiled kernel's half-range instances of every 1-qubit class: at the
+    smallest size that runs half, without the register kernel."""
+    n = 10
+    circ = W.table_mix(n, 20, seed=4) + W.layered_u3_cx(n, 30, seed=4)
+    out = []
+    for hermitian in (1, 0):
+        with engine.Simulation(n, mode="plain", plain_arith=arith, direct1=False) as s:
+            s.set_option(engine.OPT_HERMITIAN, hermitian)
+            s.extend(circ)
+            for q in range(n):
+                s.append_noise("depolarizing", (q,), 0.01)
+            s.upload()
+            s.run()
+            out.append(s.get_dm())
+    for a, b in zip(*out):
+        assert np.abs(a - b).max() <= (1e-12 if arith == "fp64" else 1e-10)
