@@ -60,6 +60,7 @@ struct dmsim_batch {
   uint64_t n_passes = 0, n_basic = 0;
   double bytes = 0, last_ms = 0;
   std::vector<std::vector<PassSpec>> plans;
+  std::vector<uint32_t> basics_of;  // basic gates of each circuit
   // tile shape: circuits of at most small_n qubits get log2(groups per tile)
   // reduced by g_shift (smaller tiles, more blocks on a small state)
   int small_n = 0, g_shift = 0;
@@ -135,7 +136,10 @@ dmsim_handle wide_sim(dmsim_batch* b, int c) {
   chk(dmsim_set_option(h, DMSIM_OPT_PLAIN_ARITH, 0), "arithmetic");
   chk(dmsim_set_option(h, DMSIM_OPT_GRAPH, 0), "graph");  // its passes are captured into the batch's graph
   for (const GateRec& g : b->circ[c]) chk(dmsim_append(h, g.op, g.qb, g.theta, g.phi, g.lambda), "append");
-  chk(dmsim_upload(h), "upload");
+  // the greedy and the plain plan are the batch's own; the learned planner
+  // also weighs the tensor cores here
+  if (b->mode == 0 || b->planner == 0) chk(sim_upload_plan(h, b->plans[c], b->basics_of[c]), "upload");
+  else chk(dmsim_upload(h), "upload");
   b->sims[c] = h;
   return h;
 }
@@ -292,8 +296,9 @@ void build(dmsim_batch* b) {
 void upload(dmsim_batch* b) {
   if (b->uploaded) throw BErr{DMSIM_ERR_STATE, "upload() called twice"};
   const int nc = (int)b->nq.size();
-  // plan every circuit (the wide ones are planned again by their engine handles)
+  // plan every circuit
   std::vector<std::vector<PassSpec>> plans(nc);
+  b->basics_of.assign(nc, 0);
   b->n_basic = 0;
   const int arith = df64_queue(b) ? AR_DF64 : AR_FP64;
   for (int c = 0; c < nc; c++) {
@@ -311,6 +316,7 @@ void upload(dmsim_batch* b) {
       plans[c] = plan_learned(basics, (int)b->nq[c], b->maxk, arith, false, m, nullptr, err);
       if (!err.empty()) throw BErr{DMSIM_ERR_CUDA, err};
     } else plans[c] = plan_greedy(basics, b->maxk);
+    b->basics_of[c] = (uint32_t)basics.size();
     b->n_basic += basics.size();
   }
   b->plans = std::move(plans);

@@ -84,13 +84,20 @@ cudaError_t launch_pass(const LaunchArgs& a, cudaStream_t s) {
 }
 
 template <typename T, int K, int CLS>
-static int occ_one() {
+static int occ_query() {
   constexpr int D = 1 << K;
   int nb = 0;
   const size_t smem = pass_smem_bytes<T, K, CLS>(kThreads * D);
   if (configure_pass<T, K, CLS, false>() != cudaSuccess) return 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pass<T, K, CLS, false>, kThreads, smem) != cudaSuccess) return 1;
   return nb > 0 ? nb : 1;
+}
+// Asked once per instance and process: an upload asks for every pass, and the
+// attribute calls and the query took 6 us each time.
+template <typename T, int K, int CLS>
+static int occ_one() {
+  static const int nb = occ_query<T, K, CLS>();
+  return nb;
 }
 
 template <typename T, int K>

@@ -11,6 +11,11 @@ namespace dmg {
 // ---------------------------------------------------------------- fusion
 namespace {
 
+// x y without std::complex's search for infinities
+cplx mul(cplx x, cplx y) {
+  return cplx(x.real() * y.real() - x.imag() * y.imag(), x.real() * y.imag() + x.imag() * y.real());
+}
+
 // Left-multiply the D x D group matrix U (qubit list qs) by basic gate b.
 void apply_basic(cplx* U, int K, const int* qs, const Basic& b) {
   const int D = 1 << K;
@@ -27,8 +32,8 @@ void apply_basic(cplx* U, int K, const int* qs, const Basic& b) {
         if (r0 & m) continue;
         const int r1 = r0 | m;
         const cplx x0 = U[r0 * D + c], x1 = U[r1 * D + c];
-        U[r0 * D + c] = b.u[0] * x0 + b.u[1] * x1;
-        U[r1 * D + c] = b.u[2] * x0 + b.u[3] * x1;
+        U[r0 * D + c] = mul(b.u[0], x0) + mul(b.u[1], x1);
+        U[r1 * D + c] = mul(b.u[2], x0) + mul(b.u[3], x1);
       }
   } else {  // BK_2Q: sub-index j = bit(q[0]) + 2 bit(q[1])
     const int i0 = pos(b.q[0]), i1 = pos(b.q[1]);
@@ -41,7 +46,7 @@ void apply_basic(cplx* U, int K, const int* qs, const Basic& b) {
         for (int j = 0; j < 4; j++) x[j] = U[rr[j] * D + c];
         for (int j = 0; j < 4; j++) {
           cplx acc = 0;
-          for (int k = 0; k < 4; k++) acc += b.u[j * 4 + k] * x[k];
+          for (int k = 0; k < 4; k++) acc += mul(b.u[j * 4 + k], x[k]);
           U[rr[j] * D + c] = acc;
         }
       }
@@ -272,13 +277,20 @@ std::vector<PassSpec> plan_greedy(const std::vector<Basic>& basics, int maxk, in
       bool grown = false;
       for (int key : cand) {
         const int j = key % m;
-        PassSpec trial = p;
         const Basic& b = basics[j];
-        add_qubit(trial, b.q[0]);
-        if (nq(b) == 2) add_qubit(trial, b.q[1]);
-        apply_basic(trial.U, trial.K, trial.q, b);
-        if (row_cap < kMaxD && max_row_nnz(trial.U, 1 << trial.K) > row_cap) continue;
-        p = trial;
+        auto absorb = [&](PassSpec& ps) {
+          add_qubit(ps, b.q[0]);
+          if (nq(b) == 2) add_qubit(ps, b.q[1]);
+          apply_basic(ps.U, ps.K, ps.q, b);
+        };
+        if (row_cap < kMaxD) {
+          PassSpec trial = p;
+          absorb(trial);
+          if (max_row_nnz(trial.U, 1 << trial.K) > row_cap) continue;
+          p = trial;
+        } else {
+          absorb(p);
+        }
         take(j);
         members++;
         grown = true;
@@ -493,51 +505,51 @@ uint64_t build_k(const PassSpec& p, int n, PassDesc<K>* d, PassFeatures* feat, u
       op.fk[a * D + b] = fk;
     }
 
-  // run masks
-  auto run_of = [&](int a, int b) {
-    int r = 0;
-    for (int j = 0; j < h.mhi; j++) {
-      const int x = hi[j];
-      int bit = 0;
-      for (int i = 0; i < K; i++) {
-        if (x == p.q[i]) bit = (a >> i) & 1;
-        if (x == p.q[i] + n) bit = (b >> i) & 1;
+  // run masks.  The run of entry (a, b) is runk[a] | runb[b]: target bits at or
+  // above L, each from the ket or the bra index.
+  int runk[kMaxD] = {0}, runb[kMaxD] = {0};
+  for (int j = 0; j < h.mhi; j++)
+    for (int i = 0; i < K; i++)
+      for (int a = 0; a < D; a++) {
+        if (hi[j] == p.q[i]) runk[a] |= ((a >> i) & 1) << j;
+        if (hi[j] == p.q[i] + n) runb[a] |= ((a >> i) & 1) << j;
       }
-      r |= bit << j;
-    }
-    return r;
-  };
   auto row_identity = [&](const cplx* M, int a) {
     for (int c = 0; c < D; c++)
       if (M[a * D + c] != (c == a ? cplx(1, 0) : cplx(0, 0))) return false;
     return true;
   };
+  bool idu[kMaxD], idv[kMaxD];
+  uint32_t colsv[kMaxD] = {0};  // bit e of [b]: V[b][e] is not zero
+  for (int a = 0; a < D; a++) {
+    idu[a] = row_identity(p.U, a);
+    idv[a] = row_identity(p.V, a);
+    for (int j = 0; j < op.nnzb[a]; j++) colsv[a] |= 1u << op.colb[a * D + j];
+  }
   std::vector<char> st(1 << h.mhi, 0), ld(1 << h.mhi, 0);
   for (int a = 0; a < D; a++)
     for (int b = 0; b < D; b++) {
       bool changed;
       if (p.cls == CLS_RLIN || p.cls == CLS_SUPER) changed = true;
       else if (mono) changed = src[a] != a || srcb[b] != b || op.fk[a * D + b] != FK_ONE;
-      else changed = !(row_identity(p.U, a) && row_identity(p.V, b));
-      if (changed) st[run_of(a, b)] = 1;
+      else changed = !(idu[a] && idv[b]);
+      if (changed) st[runk[a] | runb[b]] = 1;
     }
-  for (int a = 0; a < D; a++)
+  uint32_t from[kMaxD] = {0};  // bit e of [c]: entry (c, e) feeds a stored run
+  for (int a = 0; a < D; a++) {
+    uint32_t e = 0;  // the bra indices that row a's stored entries read
     for (int b = 0; b < D; b++) {
-      if (!st[run_of(a, b)]) continue;
-      ld[run_of(a, b)] = 1;
-      if (p.cls == CLS_RLIN || p.cls == CLS_SUPER) {
-        for (int a2 = 0; a2 < D; a2++)
-          for (int b2 = 0; b2 < D; b2++) ld[run_of(a2, b2)] = 1;
-      } else if (mono) {
-        ld[run_of(src[a], srcb[b])] = 1;
-      } else {
-        for (int c = 0; c < D; c++) {
-          if (p.U[a * D + c] == cplx(0, 0)) continue;
-          for (int e = 0; e < D; e++)
-            if (p.V[b * D + e] != cplx(0, 0)) ld[run_of(c, e)] = 1;
-        }
-      }
+      if (!st[runk[a] | runb[b]]) continue;
+      ld[runk[a] | runb[b]] = 1;
+      if (mono) ld[runk[src[a]] | runb[srcb[b]]] = 1;
+      else e |= colsv[b];
     }
+    if (!mono)
+      for (int j = 0; j < op.nnz[a]; j++) from[op.col[a * D + j]] |= e;
+  }
+  for (int c = 0; c < D; c++)
+    for (int e = 0; e < D; e++)
+      if ((from[c] >> e) & 1) ld[runk[c] | runb[e]] = 1;
   // DENSE and RLIN multiply every entry of a column, structural zeros
   // included, so every run is loaded: an unloaded run would feed
   // uninitialised shared memory (possibly NaN, and 0*NaN = NaN) into stored
