@@ -3,8 +3,8 @@
 // Life cycle as DM-Sim's Simulation (src/dmsim_nvgpu_omp.cuh:193-814):
 // append() collects gates, upload() decomposes them into basic gates, plans
 // the passes (one per basic gate in plain mode, fused k<=4 operators in fused
-// mode) and writes all pass descriptors to the device in one copy; run()
-// launches them, from its second call on by a CUDA graph.  rho stays resident
+// mode), writes all pass descriptors to the device in one copy and captures
+// the launch sequence in a CUDA graph; run() replays it.  rho stays resident
 // in HBM across runs (chained circuits), in the reference's result layout.
 #include <cuda_runtime.h>
 
@@ -76,7 +76,6 @@ struct dmsim_sim {
   size_t desc_bytes = 0;
   uint32_t n_basic = 0;
   cudaGraphExec_t gexec = nullptr;
-  uint64_t runs = 0;        // of the uploaded plan
 
   int mode = 0, maxk = 4, planner = 0, record = 0, graph_on = 1, verbose = 0;
   int fused_arith = 0;  // fused FP64 runs: FP64 width (0: FP64-width tensor passes, FP64 elsewhere) or double-float (1)
@@ -351,6 +350,27 @@ size_t plan_half_ranges(dmsim_sim* s, const std::vector<HalfCost>& costs,
   return total;
 }
 
+// The pass sequence as a graph that run() replays: also the first run, whose
+// passes, launched one by one, take 5 us each of the host.
+void capture_passes(dmsim_sim* s) {
+  cudaGraph_t graph = nullptr;
+  DM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+  try {
+    enqueue_passes(s, false, s->stream);
+  } catch (...) {
+    cudaStreamEndCapture(s->stream, &graph);
+    if (graph) cudaGraphDestroy(graph);
+    throw;
+  }
+  DM_CUDA(cudaStreamEndCapture(s->stream, &graph));
+  cudaError_t e = cudaGraphInstantiate(&s->gexec, graph, 0);
+  cudaGraphDestroy(graph);
+  if (e != cudaSuccess) {
+    s->gexec = nullptr;
+    throw DmError{DMSIM_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)};
+  }
+}
+
 // Write the descriptors of a plan to the device and capture its launches.
 void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_basic, int arith) {
   ensure_state(s);
@@ -475,29 +495,8 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     DM_CUDA(cudaStreamSynchronize(s->stream));
   }
   s->desc_bytes = total;
-  s->runs = 0;
+  if (s->graph_on && !s->passes.empty()) capture_passes(s);
   s->uploaded = true;
-}
-
-// The pass sequence as a graph that run() replays, captured by the second run
-// of a plan: one that runs only once is cheaper launched as it is.
-void capture_passes(dmsim_sim* s) {
-  cudaGraph_t graph = nullptr;
-  DM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  try {
-    enqueue_passes(s, false, s->stream);
-  } catch (...) {
-    cudaStreamEndCapture(s->stream, &graph);
-    if (graph) cudaGraphDestroy(graph);
-    throw;
-  }
-  DM_CUDA(cudaStreamEndCapture(s->stream, &graph));
-  cudaError_t e = cudaGraphInstantiate(&s->gexec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) {
-    s->gexec = nullptr;
-    throw DmError{DMSIM_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)};
-  }
 }
 
 void run(dmsim_sim* s) {
@@ -523,8 +522,6 @@ void run(dmsim_sim* s) {
     }
   }
   if (!s->keeps_herm) s->herm_known = false;
-  if (s->graph_on && !timed && !s->gexec && s->runs > 0 && !s->passes.empty()) capture_passes(s);
-  s->runs++;
   if (timed) {
     for (PassInfo& p : s->passes) {
       if (!p.ev0) DM_CUDA(cudaEventCreate(&p.ev0));

@@ -40,7 +40,7 @@ enum dmsim_option {
   DMSIM_OPT_PLANNER = 4,    /* 0 = greedy fixed width [0], 1 = learned cost model */
   DMSIM_OPT_RECORD = 5,     /* 1 = time every pass of the next runs (no graph) [0] */
   DMSIM_OPT_SEED = 6,       /* seed of measure() without uniforms; -1 = time(0) like the reference [-1] */
-  DMSIM_OPT_GRAPH = 7,      /* 1 = replay uploaded circuits from a CUDA graph, captured by the second run [1] */
+  DMSIM_OPT_GRAPH = 7,      /* 1 = replay uploaded circuits from a captured CUDA graph [1] */
   DMSIM_OPT_VERBOSE = 8,    /* 1 = print the reference's per-run timing banner [0] */
   DMSIM_OPT_FUSED_ARITH = 9, /* fused FP64 runs: 0 = FP64 width [0] (3/4-qubit passes on the tensor cores with
                                  7 BF16 digits per operand and exact integer sums, the rest in FP64), 1 = double-float
