@@ -33,7 +33,7 @@ struct dmsim_batch {
   std::vector<std::vector<GateRec>> circ;
   int mode = 1, maxk = 4, planner = 0;
   int fused_arith = 0;  // fused batches: 0 = FP64 width (the engine's default), 1 = double-float
-  int wide_n = 10;      // circuits of at least wide_n qubits run on the engine's own pass kernels
+  int wide_n = 0;       // circuits of at least wide_n qubits run on the engine's own pass kernels; 0: default_wide at upload()
   std::vector<dmsim_handle> sims;       // per circuit: the engine handle of a wide circuit, else null
   std::vector<cudaStream_t> side;       // side streams of the wide circuits' graph branches
   std::vector<cudaEvent_t> join;        // one per side stream
@@ -293,9 +293,26 @@ void build(dmsim_batch* b) {
   }
 }
 
+// From how many qubits on a circuit is a wide one.  A circuit of the 4-layer
+// ansatz takes, among many (wide, work queue): 6 qubits 10.3 and 2.6 us, 7 qubits
+// 11 and 12, 8 qubits 17 and 65, 9 qubits 77 and 311 -- and the queue's chain of
+// passes 0.45 ms at 6 qubits, so a few 6-qubit circuits are better off wide too (8
+// of them 0.09 and 0.45 ms).  More of them would be up to 64 (0.60 and 0.71 ms), but
+// a wide circuit also costs 0.3 ms more to upload.  Gate by gate, 32 circuits: 6
+// qubits 0.77 ms wide, 0.34 in the queue, 7 qubits 0.94 and 1.38; double-float: 7
+// qubits 0.41 and 0.30, 8 qubits 0.41 and 0.56.
+int default_wide(const dmsim_batch* b) {
+  if (b->mode == 0) return 7;
+  if (b->fused_arith) return 8;
+  int six = 0;
+  for (uint32_t n : b->nq) six += n == 6;
+  return six <= 8 ? 6 : 7;
+}
+
 void upload(dmsim_batch* b) {
   if (b->uploaded) throw BErr{DMSIM_ERR_STATE, "upload() called twice"};
   const int nc = (int)b->nq.size();
+  if (b->wide_n == 0) b->wide_n = default_wide(b);
   // plan every circuit
   std::vector<std::vector<PassSpec>> plans(nc);
   b->basics_of.assign(nc, 0);

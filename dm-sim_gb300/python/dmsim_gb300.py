@@ -510,7 +510,7 @@ def probe_rates():
 class Batch:
     """Many independent circuits (1..16 qubits each, uneven counts allowed),
     each from |0..0><0..0|, run together from one captured CUDA graph: the
-    circuits below ``wide_qubits`` (default 10) by one persistent work-queue
+    circuits below ``wide_qubits`` (by default the engine's rule) by one persistent work-queue
     kernel, each wider one by the engine's own pass kernels on a concurrent
     branch.  Outputs per circuit: the diagonal and <Z_i Z_{i+1}>."""
 

@@ -131,3 +131,21 @@ def test_dependency_wait_runs_out_and_gpu_stays_usable(engine):
             s.upload()
             s.run()
             assert np.abs(s.get_diag() - b.diag(0)).max() <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,arith,tol", [("fused", "fp64", 1e-12), ("fused", "df64", 1e-10), ("plain", "fp64", 1e-12)])
+@pytest.mark.parametrize("six", [3, 9])
+def test_default_line_between_wide_and_narrow(engine, oracle, mode, arith, tol, six):
+    """Circuits on either side of every default line, with few and with many
+    6-qubit ones, against the statevector oracle."""
+    rng = np.random.default_rng(six)
+    sweep = [(6, W.hea(6, 1, rng)) for _ in range(six)] + [(n, W.hea(n, 2, rng)) for n in (1, 2, 5, 7, 8, 9, 10)]
+    with engine.Batch([n for n, _ in sweep], mode=mode, fused_arith=arith) as b:
+        for c, (_, circ) in enumerate(sweep):
+            b.extend(c, circ)
+        b.upload()
+        b.run()
+        for c, (n, circ) in enumerate(sweep):
+            sr, si = oracle.sv_sim(n, circ)
+            assert np.abs(b.diag(c) - (sr ** 2 + si ** 2)).max() <= tol
