@@ -7,18 +7,17 @@
 // V's.  Every FP32 operand value is the sum of three BF16 values, each
 // rounded from the remainder of the ones before it (x = h + m + l to 2^-24
 // of |x|; the host split W and V's entries the same way, slices 0..2 of
-// TcDesc).  The six products whose size reaches 2^-16 of the leading one --
-// (l,h) (m,m) (h,l), then (m,h) (h,m), then (h,h), smallest first --
-// accumulate into one FP32 accumulator in tensor memory; the three dropped
-// ones are below 2^-24 of it.  Each value keeps its own 24-bit precision
+// TcDesc).  The six products whose size reaches 2^-16 of the leading one
+// accumulate into three FP32 accumulators in tensor memory -- (h,h); (h,m) and
+// (m,h); (h,l), (m,m) and (l,h) -- which are added in FP32, the small ones
+// first; the three dropped products are below 2^-24 of the leading one.  Each value keeps its own 24-bit precision
 // (no shared exponent per column), so a step's error is FP32 accumulation's,
 // the FP32-pipe passes' own level.
 //
 // Threads, tiles and synchronisation follow tensor64.cu: 512 threads, two
-// blocks per SM (64 registers a thread, 107 KB of shared memory and 64 TMEM
+// blocks per SM (64 registers a thread, 107 KB of shared memory and 256 TMEM
 // columns a block), two independent groups of 8 warps taking alternate tiles,
-// each with its own tile buffer (1-D TMA bulk copies of the tile's runs, issued
-// one tile ahead), slice operand, accumulator (R TMEM columns), mbarriers and
+// each with its own tile buffer (filled one tile ahead), slice operand, accumulators (3 R TMEM columns), mbarriers and
 // named barrier.  Per tile:
 //   1. wait for the tile, ket slices -> A;  2. the ket MMAs;  3. ket
 //      accumulator -> FP32 ket outputs in place of the tile;  4. bra slices
@@ -29,6 +28,11 @@
 // barrier, waits (bounded) for its own copies and MMAs in flight, sets the
 // error flag, and the block releases its tensor memory; the host reports
 // DMSIM_ERR_TIMEOUT with rho undefined.
+//
+// What bounds it: issue (60 % active), the ALU and the load/store pipe (40 %
+// each).  A 4-qubit pass at 15 qubits (8.6 GB read and as much written) takes
+// 4.7 ms, 3.7 TB/s; 6.6 ms before the tiles came in by 16-byte copies (5.1) and
+// the orders had accumulators of their own (4.8).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -57,22 +61,21 @@ struct T32 {
   static constexpr uint32_t SBO = 16 * R;                  // bytes between 8-row groups of an R-wide operand
   static constexpr uint32_t A_BYTES = 128 * R * 2;         // one slice of the 128 columns
   static constexpr uint32_t B_BYTES = R * R * 2;           // one slice of W or V
-  static constexpr uint32_t SET_COLS = R;                  // the accumulator of one group
-  static constexpr uint32_t TMEM_COLS = 2 * SET_COLS;      // 64 (K = 4), 32 (K = 3)
-  static constexpr uint32_t TX_BYTES = TILE * 4 * 2;       // one tile, re + im
+  static constexpr uint32_t SET_COLS = 3 * R;              // the accumulators of one group, an order each
+  static constexpr uint32_t TMEM_COLS = 8 * R;             // two sets, a power of two: 256 (K = 4), 128 (K = 3)
   static constexpr uint32_t BUF_BYTES = 2 * ASTR * 4;      // one group's tile buffer
   static_assert(ASTR % 32 == 16 && BUF_BYTES % 16 == 0, "tile buffer layout");
-  static_assert(TMEM_COLS <= 512, "two accumulator sets must fit in tensor memory");
+  static_assert(2 * TMEM_COLS <= 512, "two blocks of two accumulator sets in tensor memory");
 };
 
 // Shared-memory position of local entry e of a loaded tile: 16-entry pieces
-// 20 entries apart (each piece's destination 16-byte aligned for the bulk
-// copies).  Additive over disjoint bit fields.
+// 20 entries apart (16-byte chunks stay aligned).  Additive over disjoint bit fields.
 __device__ __forceinline__ int piece_off32(int e) { return e + 4 * (e >> 4); }
 
 struct T32Group {
   uint64_t full;  // the group's tile loads
   uint64_t mma;   // the group's ket and bra commits, alternating
+  uint64_t nbase; // global index of the group's next tile
 };
 
 template <int K>
@@ -137,29 +140,37 @@ __device__ __forceinline__ void slice_column(const float (&v)[D], int row, int h
   }
 }
 
-// This warp's D consecutive TMEM columns (32 lanes) in one load.
-template <int D>
-__device__ __forceinline__ void tmem_ld_row(uint32_t taddr, float (&v)[D]) {
-  if constexpr (D == 16) tc::tmem_ld16(taddr, v);
-  else tc::tmem_ld8(taddr, v);
+// Eight consecutive outputs of this warp's 32 rows: the three orders, the
+// small ones first.
+__device__ __forceinline__ void sum_orders8(uint32_t taddr, uint32_t r, float (&v)[8]) {
+  float o1[8], o2[8];
+  tc::tmem_ld8(taddr, v);
+  tc::tmem_ld8(taddr + r, o1);
+  tc::tmem_ld8(taddr + 2 * r, o2);
+  tc::tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < 8; c++) v[c] = __fadd_rn(v[c], __fadd_rn(o1[c], o2[c]));
 }
 
-// One thread issues every product of a step: slice pairs (i of the columns,
-// j of the operator) (2,0) (1,1) (0,2) (1,0) (0,1) (0,0), smallest first,
-// all into the group's one accumulator (N = R).
+// One thread issues every product of a step: slice i of the columns against
+// the operator's slices 0..2-i, which are consecutive blocks of one operand, so
+// that the pairs of order i + j meet in the accumulator of order i + j: (0; 0,
+// 1, 2), (1; 0, 1), (2; 0).  Six MMAs of N = 3R, 2R and R instead of twelve of N
+// = R (a small MMA takes about 140 cycles whatever its N), and the leading
+// products (16 bits) keep FP32 accumulators of their own, without the
+// truncation of sums of all orders.
 template <int K>
 __device__ __forceinline__ void issue_step32(const unsigned char* sA, const unsigned char* sBside, uint32_t dset) {
   using S = T32<K>;
   constexpr int R = S::R;
   const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sBside);
-  constexpr int kPairs[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-  for (int q = 0; q < 6; q++) {
+  for (int i = 0; i < kT32Slices; i++) {
 #pragma unroll
     for (int kk = 0; kk < R / 16; kk++) {
-      const uint64_t ad = tc::smem_desc(a0 + kPairs[q][0] * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
-      const uint64_t bd = tc::smem_desc(b0 + kPairs[q][1] * S::B_BYTES + kk * 256, tc::kLbo, S::SBO);
-      tc::mma_f16kind(dset, ad, bd, tc::idesc_bf16_f32(128, R), (q == 0 && kk == 0) ? 0u : 1u);
+      const uint64_t ad = tc::smem_desc(a0 + i * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
+      const uint64_t bd = tc::smem_desc(b0 + kk * 256, tc::kLbo, S::SBO);
+      tc::mma_f16kind(dset + i * R, ad, bd, tc::idesc_bf16_f32(128, (kT32Slices - i) * R), (i == 0 && kk == 0) ? 0u : 1u);
     }
   }
 }
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(kT32Threads, 2)
   }
   if (tid == 0) {
     for (int gi = 0; gi < 2; gi++) {
-      tc::mbar_init(&tb.grp[gi].full, 1);
+      tc::mbar_init(&tb.grp[gi].full, kT32GroupThreads);
       tc::mbar_init(&tb.grp[gi].mma, 1);
     }
     tc::mbar_fence_init();
@@ -266,11 +277,10 @@ __global__ void __launch_bounds__(kT32Threads, 2)
   };
   const int lf = free_off(f);  // accumulator steps: free offset of column (., f) in the state
   // slice steps: column (b = rc, fc)'s values a = 0..D-1 of half hc at
-  // buf[basec + tb.pk[a]] (the offsets read from shared memory, a broadcast,
-  // to keep the register budget of two blocks per SM)
+  // buf[basec + the strides tb.pk[1, 2, 4, 8] of a's bits]
   const int basec = hc * ASTR + tb.pb[rc] + piece_off32(free_off(fc));
   const uint64_t ntiles = h.ntiles, gstep = 2 * (uint64_t)gridDim.x;
-  const int runlen = 1 << L, lgp = L < 4 ? L : 4, npieces = (2 * TILE) >> lgp;
+  const int runlen = 1 << L;
   // The ket step's outputs Y(a, b) of column (b, ff) replace the tile in its
   // buffer, at [hh][a][b ^ (a & 1)][ff]: the ket step writes, for one a, 32
   // consecutive words per warp, and the bra step reads, for one b, columns a
@@ -285,18 +295,22 @@ __global__ void __launch_bounds__(kT32Threads, 2)
     return base;
   };
 
-  // Loads of a tile into the group's buffer: the group's first thread arms
-  // its barrier with the tile's bytes before a group barrier, after which
-  // every thread of the group issues its share of the 1-D bulk copies, one
-  // per piece (16 entries, or a whole run when runs are shorter) of each
-  // array.  Runs are at least 8 entries (32 bytes) long.
+  // Loads of a tile into the group's buffer, by every thread of the group
+  // after a group barrier that frees it: 16-byte asynchronous copies (runs are
+  // at least 8 entries long), each thread's arriving on the group's barrier
+  // when they have landed.  With 1-D bulk copies of 64 bytes, each issued for
+  // 90 cycles or so, and every thread finding the next tile, this step took
+  // half of a tile's time.
   auto copy_tile = [&](uint64_t base) {
-    for (int i = gtid; i < npieces; i += kT32GroupThreads) {
-      const int arr = i & 1, e0 = (i >> 1) << lgp;
-      const int run = e0 >> L, o = e0 & (runlen - 1);
-      tc::bulk_g2s(buf + arr * ASTR + piece_off32(e0), (arr ? im : re) + base + tb.hioff[run] + o, 4u << lgp,
-                   &gp.full);
+#pragma unroll
+    for (int k = 0; k < TILE / 4 / kT32GroupThreads; k++) {
+      const int e0 = 4 * (gtid + k * kT32GroupThreads);
+      const uint64_t src = base + tb.hioff[e0 >> L] + (uint64_t)(e0 & (runlen - 1));
+      float* dst = buf + piece_off32(e0);
+      tc::cp_async16(dst, re + src);
+      tc::cp_async16(dst + ASTR, im + src);
     }
+    tc::cp_async_arrive(&gp.full);
   };
 
   // outstanding asynchronous work of this thread's view; a phase that did not
@@ -317,8 +331,6 @@ __global__ void __launch_bounds__(kT32Threads, 2)
   // ---- prologue: the group's first tile in flight
   uint64_t t = blockIdx.x + (uint64_t)g * gridDim.x;
   uint64_t tbase = t < ntiles ? tile_base_s(t) : 0;
-  if (gtid == 0 && t < ntiles) tc::mbar_arrive_expect_tx(&gp.full, S::TX_BYTES);
-  group_bar32(g);
   if (t < ntiles) {
     copy_tile(tbase);
     pendf = 1;
@@ -329,8 +341,10 @@ __global__ void __launch_bounds__(kT32Threads, 2)
     wait(&gp.full, phf, pendf);
     {
       float v[D];
+      const int p1 = tb.pk[1], p2 = tb.pk[2], p4 = tb.pk[4], p8 = tb.pk[D / 2];
 #pragma unroll
-      for (int a = 0; a < D; a++) v[a] = buf[basec + tb.pk[a]];
+      for (int a = 0; a < D; a++)
+        v[a] = buf[basec + (a & 1 ? p1 : 0) + (a & 2 ? p2 : 0) + (a & 4 ? p4 : 0) + (a & 8 ? p8 : 0)];
       slice_column<D, S::A_BYTES, S::SBO>(v, mc, hc, sA);
     }
     tc::fence_proxy_async_smem();
@@ -344,15 +358,21 @@ __global__ void __launch_bounds__(kT32Threads, 2)
       tc::mma_commit(&gp.mma);
     }
     pendm = 1;
+    const uint64_t tn = t + gstep;
+    // one thread finds the group's next tile while the products run (every
+    // thread reads it in step 5, two barriers on)
+    if (gtid == kT32GroupThreads - 1 && tn < ntiles) gp.nbase = tile_base_s(tn);
 
     // ---- 3: ket outputs of column (b = r, f), in place of the tile
     if (wait(&gp.mma, phm, pendm)) {
       tc::fence_after_sync();
-      float sv[D];
-      tmem_ld_row<D>(tmem + tlane + half * D, sv);
-      tc::tmem_wait_ld();
 #pragma unroll
-      for (int a = 0; a < D; a++) buf[yoff(half, a, r, f)] = sv[a];
+      for (int a0 = 0; a0 < D; a0 += 8) {
+        float sv[8];
+        sum_orders8(tmem + tlane + half * D + a0, R, sv);
+#pragma unroll
+        for (int a = 0; a < 8; a++) buf[yoff(half, a0 + a, r, f)] = sv[a];
+      }
     }
     tc::fence_before_sync();
     if (group_bar_or32(g, bad)) break;
@@ -365,8 +385,6 @@ __global__ void __launch_bounds__(kT32Threads, 2)
       for (int b = 0; b < D; b++) v[b] = buf[yoff(hc, rc, b, fc)];
       slice_column<D, S::A_BYTES, S::SBO>(v, mc, hc, sA);
     }
-    const uint64_t tn = t + gstep;
-    if (gtid == 0 && tn < ntiles) tc::mbar_arrive_expect_tx(&gp.full, S::TX_BYTES);  // the group's next tile
     tc::fence_proxy_async_smem();
     tc::fence_before_sync();
     group_bar32(g);
@@ -378,7 +396,7 @@ __global__ void __launch_bounds__(kT32Threads, 2)
       tc::mma_commit(&gp.mma);
     }
     pendm = 1;
-    const uint64_t nbase = tn < ntiles ? tile_base_s(tn) : 0;
+    const uint64_t nbase = gp.nbase;
     if (tn < ntiles) {
       copy_tile(nbase);
       pendf = 1;
@@ -388,19 +406,22 @@ __global__ void __launch_bounds__(kT32Threads, 2)
     if (wait(&gp.mma, phm, pendm)) {
       tc::fence_after_sync();
       float* arr = (half ? im : re) + tbase + lf;
-      float sv[D];
-      tmem_ld_row<D>(tmem + tlane + half * D, sv);
-      tc::tmem_wait_ld();
-      if (tb.allstored) {  // the common case: one base per thread, one offset per output
-        float* col = arr + tb.offk[r];
 #pragma unroll
-        for (int b = 0; b < D; b++) col[tb.offb[b]] = sv[b];
-      } else {
+      for (int b0 = 0; b0 < D; b0 += 8) {
+        float sv[8];
+        sum_orders8(tmem + tlane + half * D + b0, R, sv);
+        if (tb.allstored) {  // the common case
+          float* col = arr + tb.offk[r] + tb.offb[b0];
+          const uint64_t s1 = tb.offb[1], s2 = tb.offb[2], s4 = tb.offb[4];
 #pragma unroll
-        for (int b = 0; b < D; b++) {
-          const uint64_t T = tb.outoff[b][r];
-          if (!(T >> 63)) continue;  // a run the pass does not change
-          arr[T & 0xFFFFFFFFFFFFull] = sv[b];
+          for (int b = 0; b < 8; b++) col[(b & 1 ? s1 : 0) + (b & 2 ? s2 : 0) + (b & 4 ? s4 : 0)] = sv[b];
+        } else {
+#pragma unroll
+          for (int b = 0; b < 8; b++) {
+            const uint64_t T = tb.outoff[b0 + b][r];
+            if (!(T >> 63)) continue;  // a run the pass does not change
+            arr[T & 0xFFFFFFFFFFFFull] = sv[b];
+          }
         }
       }
     }
