@@ -132,14 +132,33 @@ __device__ __forceinline__ bool named_bar_or(int id, bool p) {
   return r != 0;
 }
 
-// ---- MMA: D[tmem] (+)= A[smem] * B[smem]^T, one thread issues; kind::f16 (the descriptor says FP16 or BF16)
+// 1 in one lane of a converged warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
+}
+
+// ---- MMA: D[tmem] (+)= A[smem] * B[smem]^T; kind::f16 (the descriptor says FP16
+// or BF16), by one thread
 __device__ __forceinline__ void mma_f16kind(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
+                                            uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same run by a whole warp, issued by the lane with `elected`.
+__device__ __forceinline__ void mma_f16kind_if(uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                               uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 // Arrive on the mbarrier once every MMA this thread issued so far completes.

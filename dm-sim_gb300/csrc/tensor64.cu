@@ -38,7 +38,7 @@
 // + (l & 7) and quarter l >> 3 of it (half l >> 4, values (l >> 3) & 1 of
 // that half; the four quarters of a column in one warp); in the accumulator
 // steps column m = 32 (w & 3) + l -- the TMEM lane quadrant its warp may read
-// -- and quarter ((w & 15) >> 2).  The group's first thread issues its MMAs.
+// -- and quarter ((w & 15) >> 2).  The group's first warp issues its MMAs.
 // Per tile:
 //   1. wait for the tile (copied one tile ahead), column maxima, ket digits
 //      -> A;  2. the ket MMAs;  3. ket accumulators -> exact int64 outputs in
@@ -54,7 +54,7 @@
 // What bounds it: the ALU, the FP64 pipe's conversions and shared memory are
 // each near half busy; a group's steps follow one another, and tensor memory
 // and the digit operands leave room for two groups.  A 4-qubit pass over half
-// of a 14-qubit state (2.2 GB read, 2.2 written) takes 2.1 ms, of which a
+// of a 14-qubit state (2.2 GB read, 2.2 written) takes 1.93 ms, of which a
 // group spends about a fifth on each of: ket digits, MMAs, outputs.  It took
 // 2.6 ms with the digits converted to BF16 one by one and the sums taken apart
 // by an FP32 addition each (156 against 224 instructions a value, now fewer).
@@ -168,7 +168,7 @@ constexpr uint64_t kDigitBias = 0x0080808080808080ull;
 // subnormals become numbers below 2^-9, hence 0); grids of 2^1077 and above,
 // where the exponent field could wrap, shift the significand instead.  Without
 // kConvert all do, on the ALU, towards zero.  Three values in four convert: a
-// 4-qubit pass at 14 qubits takes 2100 us, with all 2170, half 2240, none 2430.
+// 4-qubit pass at 14 qubits took 2100 us, with all 2170, half 2240, none 2430.
 template <bool kConvert>
 __device__ __forceinline__ int64_t align_fp64(uint32_t lo, uint32_t hi, uint32_t ecm) {
   if (kConvert && ecm < (1077u << 20)) {
@@ -262,34 +262,35 @@ __device__ __forceinline__ int leading_bit(int32_t x) {
   return r;
 }
 
-// One thread issues every product of a step: digit slices A_0..A_6 of the
+// The group's first warp issues every product of a step, by its elected lane: digit slices A_0..A_6 of the
 // 128 columns against the operator's slices, slice pairs of orders 0..7, the
 // pairs of order o into the accumulator at TMEM column o*R of the set.  The
 // operator's slices are consecutive R-row blocks of one K-major operand, so
 // A_i against slices j0..j0+nb-1 is one MMA of N = nb*R.  The first product
 // (128 columns of ones against three FP16 numbers a row, TcDesc64::start) sets
 // every accumulator to 0.75 - 128 2^-24 sum w: the digits' excess of 128 taken
-// off, and a sum whose FP32 bits are an integer (kAcc0 + S).
+// off, and a sum whose FP32 bits are an integer (kAcc0 + S).  The warp stays
+// together and one lane issues: with the addresses worked out in one lane's
+// branch an MMA took 140 cycles, more than it runs, and a pass 2.10 ms for 1.93.
 template <int K>
 __device__ __forceinline__ void issue_step(const unsigned char* sA, const unsigned char* sBside,
-                                           const unsigned char* sAI, const unsigned char* sBI, uint32_t dset) {
+                                           const unsigned char* sAI, const unsigned char* sBI, uint32_t dset,
+                                           uint32_t elected) {
   using S = T64<K>;
   constexpr int R = S::R;
   const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sBside);
   // K columns 8..15: A's zeros, 128 rows (2 KB) on; B's are whatever finite
   // numbers follow the row group (the next rows' or side's, or A's ones)
-  tc::mma_f16kind(dset, tc::smem_desc(tc::smem_u32(sAI), 2048, 128), tc::smem_desc(tc::smem_u32(sBI), 128, 128),
-               tc::idesc_f16_f32(128, kTc64Orders * R), 0u);
-  auto issue = [&](int i, int j0, int nb) {
+  tc::mma_f16kind_if(elected, dset, tc::smem_desc(tc::smem_u32(sAI), 2048, 128),
+                     tc::smem_desc(tc::smem_u32(sBI), 128, 128), tc::idesc_f16_f32(128, kTc64Orders * R), 0u);
 #pragma unroll
-    for (int kk = 0; kk < R / 16; kk++) {
-      const uint64_t ad = tc::smem_desc(a0 + i * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
-      const uint64_t bd = tc::smem_desc(b0 + j0 * S::B_BYTES + kk * 256, tc::kLbo, S::SBO);
-      tc::mma_f16kind(dset + (i + j0) * R, ad, bd, tc::idesc_f16_f32(128, nb * R), 1u);
-    }
-  };
+  for (int i = 0; i < kTc64Slices; i++) {
+    const int nb = i == 0 ? kTc64Slices : kTc64Orders - i;  // (i, 0..6 or 7-i)
 #pragma unroll
-  for (int i = 0; i < kTc64Slices; i++) issue(i, 0, i == 0 ? kTc64Slices : kTc64Orders - i);  // (i, 0..6 or 7-i)
+    for (int kk = 0; kk < R / 16; kk++)
+      tc::mma_f16kind_if(elected, dset + i * R, tc::smem_desc(a0 + i * S::A_BYTES + kk * 256, tc::kLbo, S::SBO),
+                         tc::smem_desc(b0 + kk * 256, tc::kLbo, S::SBO), tc::idesc_f16_f32(128, nb * R), 1u);
+  }
 }
 
 }  // namespace
@@ -521,9 +522,10 @@ __global__ void __launch_bounds__(kT64Threads, 1)
     tc::fence_after_sync();
 
     // ---- 2: ket products
-    if (gtid == 0) {
-      issue_step<K>(sA, sB, sAI, sBI, tmem);
-      tc::mma_commit(&gp.mma);
+    if (wg == 0) {
+      const uint32_t elected = tc::elect_one();
+      issue_step<K>(sA, sB, sAI, sBI, tmem, elected);
+      if (elected) tc::mma_commit(&gp.mma);
     }
     pendm = 1;
     const uint64_t tn = t + gstep;
@@ -597,9 +599,10 @@ __global__ void __launch_bounds__(kT64Threads, 1)
     tc::fence_after_sync();
 
     // ---- 5: bra products; the group's next tile into the freed buffer
-    if (gtid == 0) {
-      issue_step<K>(sA, sB + kTc64Slices * S::B_BYTES, sAI, sBI + S::BI_BYTES, tmem);
-      tc::mma_commit(&gp.mma);
+    if (wg == 0) {
+      const uint32_t elected = tc::elect_one();
+      issue_step<K>(sA, sB + kTc64Slices * S::B_BYTES, sAI, sBI + S::BI_BYTES, tmem, elected);
+      if (elected) tc::mma_commit(&gp.mma);
     }
     pendm = 1;
     const uint64_t nbase = gp.nbase;
