@@ -155,11 +155,27 @@ void check_qubits(const dmsim_sim* s, const GateRec& g) {
 // includes the mirror pass that it needs before it, the last one the mirror
 // that brings the whole state up to date.
 void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
+  // Whether the next kernel may start under the one before it (kernels.h), so
+  // that launch, tables and tensor-memory allocation overlap: states up to 12
+  // qubits (5 qubits gate by gate 1870 -> 1380 us, 8 qubits fused 565 -> 415, 12
+  // qubits fused 20.3 -> 19.9 ms; at 14 qubits the waiting blocks cost 3 %), and
+  // only grids of at most one block an SM, of whole numbers of them (persistent
+  // blocks) or of several: otherwise blocks placed around the running kernel's make
+  // uneven loads (9 qubits, 256 blocks: 565 -> 720).
+  const bool overlap = !timed && s->n <= 12;
+  auto may_overlap = [&](unsigned grid) {
+    const unsigned sms = (unsigned)s->sms;
+    return grid <= sms || grid % sms == 0 || grid >= 4 * sms;
+  };
+  bool pdl = false;  // a kernel of the sequence goes before
   auto mirror = [&](uint32_t from, uint32_t to, bool last) {
-    if (from) DM_CUDA(launch_mirror(s->d_re, s->d_im, (int)s->n, s->arith, from, to, last, s->d_herm, s->sms, st));
+    if (!from) return;
+    DM_CUDA(launch_mirror(s->d_re, s->d_im, (int)s->n, s->arith, from, to, last, s->d_herm, s->sms, pdl, st));
+    pdl = overlap;
   };
   for (size_t i = 0; i < s->passes.size(); i++) {
     PassInfo& p = s->passes[i];
+    if (p.renorm || p.conv || p.transpose) pdl = false;
     if (p.renorm) {
       if (timed) DM_CUDA(cudaEventRecord(p.ev0, st));
       DM_CUDA(launch_renormalise(s->d_re, s->d_im, (int)s->n, s->fp32, s->d_acc + 4, p.grid, st));
@@ -202,7 +218,9 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.herm = s->d_herm;
     if (timed) DM_CUDA(cudaEventRecord(p.ev0, st));
     if (p.stale != p.half) mirror(p.stale, p.half, false);
+    a.pdl = pdl && may_overlap(p.grid);
     DM_CUDA(launch_pass(a, st));
+    pdl = overlap;
     if (i + 1 == s->passes.size()) mirror(s->end_stale, 0, true);
     if (timed) DM_CUDA(cudaEventRecord(p.ev1, st));
   }

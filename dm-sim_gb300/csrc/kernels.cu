@@ -212,6 +212,8 @@ __global__ void __launch_bounds__(256) k_mirror(uint64_t* __restrict__ re, uint6
   using U = uint64_t;
   constexpr int TS = 32;
   __shared__ U s_re[TS][TS + 1], s_im[TS][TS + 1];
+  pdl_wait();
+  pdl_begin();
   if (!*herm) return;
   const uint64_t dim = 1ull << n;
   const uint32_t nt = (uint32_t)(dim / TS);
@@ -244,14 +246,13 @@ __global__ void __launch_bounds__(256) k_mirror(uint64_t* __restrict__ re, uint6
 }
 
 cudaError_t launch_mirror(void* re, void* im, int n, int arith, uint32_t from, uint32_t to, bool last,
-                          const int* herm, int sms, cudaStream_t s) {
+                          const int* herm, int sms, bool pdl, cudaStream_t s) {
   if (n < 5 || arith == AR_FP32) return cudaErrorInvalidValue;
   // an odd grid: a block's tiles then run through all the residues that the sets' bits decide by
   const uint64_t nt = 1ull << (n - 5);
   const unsigned grid = (unsigned)std::min<uint64_t>(nt * nt, (uint64_t)sms * 8 - 1);
-  k_mirror<<<grid, 256, 0, s>>>((uint64_t*)re, (uint64_t*)im, n, from, to, last,
-                                arith == AR_DF64 ? 0x8000000080000000ull : 0x8000000000000000ull, herm);
-  return cudaGetLastError();
+  return launch_kernel(pdl, k_mirror, grid, 256, 0, s, (uint64_t*)re, (uint64_t*)im, n, from, to, (int)last,
+                       arith == AR_DF64 ? 0x8000000080000000ull : 0x8000000000000000ull, herm);
 }
 
 // rho may have been written from outside (dmsim_set_dm, the device pointers),

@@ -10,7 +10,32 @@ namespace dmg {
 // Arithmetic of a pass: the state's element type.
 enum Arith : int { AR_FP64 = 0, AR_FP32 = 1, AR_DF64 = 2 };
 
+// A pass may be launched while the one before it is still running (programmatic
+// dependent launch): it finds its tables, then waits for the other's end before
+// it touches the state (pdl_wait), and only then lets the next one start
+// (pdl_begin): a chain of them stays in order, and one kernel at most waits on the
+// SMs beside the running one.
+template <typename... P, typename... A>
+cudaError_t launch_kernel(bool pdl, void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&c, k, static_cast<P>(args)...);
+}
+#if defined(__CUDACC__)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 struct LaunchArgs {
+  bool pdl;            // may start before the pass before it has ended
   void* re;            // device real parts (double, float, or double-float pairs)
   void* im;            // device imaginary parts
   const void* desc;    // device PassDesc<K>
@@ -61,7 +86,7 @@ cudaError_t launch_conj_transpose(void* re, void* im, int n, bool fp32, unsigned
 // Entries stale under `from` that `to` needs (0: every one) <- conj of their
 // transposes, if *herm.  last: also make the ties exactly Hermitian.
 cudaError_t launch_mirror(void* re, void* im, int n, int arith, uint32_t from, uint32_t to, bool last,
-                          const int* herm, int sms, cudaStream_t s);
+                          const int* herm, int sms, bool pdl, cudaStream_t s);
 // *herm <- 1 if rho (FP64 entries) equals its conjugate transpose exactly, else 0
 cudaError_t launch_check_hermitian(const void* re, const void* im, int n, int* herm, int sms, cudaStream_t s);
 cudaError_t launch_set_flag(int* flag, int value, cudaStream_t s);

@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   const uint64_t ngroups = hm ? hm->count : 1ull << (2 * n - 2);
   const uint64_t mq = 1ull << q, mb = 1ull << (q + n);
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  pdl_wait();
+  pdl_begin();
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += stride) {
     uint64_t i;
     if (hm) {
@@ -263,9 +265,8 @@ cudaError_t launch1(const LaunchArgs& a, cudaStream_t s) {
   } else if (a.half) {
     return cudaErrorInvalidValue;
   }
-  k<<<a.grid, 256, 0, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im), static_cast<const PassDesc<1>*>(a.desc), a.q0,
-                           a.n, a.half, a.herm);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k, a.grid, 256, 0, s, static_cast<T*>(a.re), static_cast<T*>(a.im),
+                       static_cast<const PassDesc<1>*>(a.desc), a.q0, a.n, a.half, a.herm);
 }
 
 template <typename T>

@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(Mono<T, K>::NT, K <= 3 ? 2 : 1)
     tc::cp_async_commit();
   };
 
+  pdl_wait();
+  pdl_begin();
   uint64_t t = blockIdx.x;
 #pragma unroll
   for (int s = 0; s < ST - 1; s++) load(t + (uint64_t)s * gridDim.x, s);
@@ -187,9 +189,8 @@ cudaError_t launch_mono_one(const LaunchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_mono<T, K, CLS><<<a.grid, M::NT, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                                static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k_mono<T, K, CLS>, a.grid, M::NT, smem, s, static_cast<T*>(a.re), static_cast<T*>(a.im),
+                       static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
 }
 
 template <typename T, int K>

@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(kThreads) k_pass(T* __restrict__ re, T* __rest
   auto& tb = *reinterpret_cast<PassTables<T, K, CLS>*>(smem_raw + ((2 * (size_t)tile * sizeof(T) + 15) & ~(size_t)15));
   load_tables<T, K, CLS>(dp, tb);
   __syncthreads();
+  pdl_wait();
+  pdl_begin();
   // Full-size tiles of narrow passes (2^(K-1) entry pairs per thread): the
   // next tile's loads go out before the current tile is transformed.
   constexpr int P = K >= 1 ? 1 << (K - 1) : 1;
@@ -96,9 +98,8 @@ inline cudaError_t launch_one(const LaunchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_pass<T, K, CLS, HALF><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                                   static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k_pass<T, K, CLS, HALF>, a.grid, kThreads, smem, s, static_cast<T*>(a.re),
+                       static_cast<T*>(a.im), static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
 }
 
 }  // namespace dmg

@@ -382,6 +382,8 @@ __global__ void __launch_bounds__(kThreads, TcMinBlocks<T>::value) k_pass_tc(T* 
   constexpr int PAIRS = SH::TILE / 2 / kThreads;
   const HalfMap* hm = hmap && *herm ? hmap : nullptr;  // the half range of the tiles, if any
   const uint64_t ntiles = hm ? hm->count : h.ntiles;
+  pdl_wait();
+  pdl_begin();
   uint64_t t = blockIdx.x;
   if (t < ntiles) {
     const uint64_t base = tile_base(h, hm, t);
@@ -466,9 +468,8 @@ static cudaError_t launch_tc_k(const LaunchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_pass_tc<K, T><<<a.grid, kThreads, smem, s>>>(static_cast<T*>(a.re), static_cast<T*>(a.im),
-                                                  static_cast<const TcDesc<K>*>(a.desc), a.err, a.half, a.herm);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k_pass_tc<K, T>, a.grid, kThreads, smem, s, static_cast<T*>(a.re), static_cast<T*>(a.im),
+                       static_cast<const TcDesc<K>*>(a.desc), a.err, a.half, a.herm);
 }
 
 cudaError_t launch_pass_tc(const LaunchArgs& a, cudaStream_t s) {

@@ -329,6 +329,8 @@ __global__ void __launch_bounds__(kT32Threads, 2)
   };
 
   // ---- prologue: the group's first tile in flight
+  pdl_wait();
+  pdl_begin();
   uint64_t t = blockIdx.x + (uint64_t)g * gridDim.x;
   uint64_t tbase = t < ntiles ? tile_base_s(t) : 0;
   if (t < ntiles) {
@@ -462,9 +464,8 @@ static cudaError_t launch_tc32_k(const LaunchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_pass_tc32<K><<<a.grid, kT32Threads, t32_smem_bytes<K>(), s>>>(
-      static_cast<float*>(a.re), static_cast<float*>(a.im), static_cast<const TcDesc<K>*>(a.desc), a.err);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k_pass_tc32<K>, a.grid, kT32Threads, t32_smem_bytes<K>(), s, static_cast<float*>(a.re),
+                       static_cast<float*>(a.im), static_cast<const TcDesc<K>*>(a.desc), a.err);
 }
 
 cudaError_t launch_pass_tc32(const LaunchArgs& a, cudaStream_t s) {

@@ -484,6 +484,8 @@ __global__ void __launch_bounds__(kT64Threads, 1)
   };
 
   // ---- prologue: the group's first tile in flight
+  pdl_wait();
+  pdl_begin();
   uint64_t t = blockIdx.x + (uint64_t)g * gridDim.x;
   uint64_t tbase = t < ntiles ? tile_base_s(t) : 0;
   if (t < ntiles) {
@@ -678,10 +680,9 @@ static cudaError_t launch_tc64_k(const LaunchArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     configured = 1;
   }
-  k_pass_tc64<K><<<a.grid, kT64Threads, t64_smem_bytes<K>(), s>>>(
-      static_cast<uint64_t*>(a.re), static_cast<uint64_t*>(a.im), static_cast<const TcDesc64<K>*>(a.desc), a.err,
-      a.half, a.herm, a.n);
-  return cudaGetLastError();
+  return launch_kernel(a.pdl, k_pass_tc64<K>, a.grid, kT64Threads, t64_smem_bytes<K>(), s, static_cast<uint64_t*>(a.re),
+                       static_cast<uint64_t*>(a.im), static_cast<const TcDesc64<K>*>(a.desc), a.err, a.half, a.herm,
+                       a.n);
 }
 
 cudaError_t launch_pass_tc64(const LaunchArgs& a, cudaStream_t s) {
