@@ -912,7 +912,7 @@ bool tc_choose(const PassSpec& p, int n, int tensor_opt, int arith) {
   if (tensor_opt == 2) return true;  // every eligible pass (measurements)
   if (p.tc >= 0) return p.tc != 0;   // the learned planner's choice
   if (arith == 0) return true;       // FP64: the alternative is GB300's FP64 pipe
-  // complex64: 4-qubit passes on the tensor cores (tensor32.cu: 3.7 TB/s at 15
+  // complex64: 4-qubit passes on the tensor cores (tensor32.cu: 3.5 TB/s at 15
   // qubits; the FP32-pipe kernel 1.8); 3-qubit ones stay on the FP32 pipe (2.9 TB/s
   // against 3.3 at 15 qubits, but 2 % slower circuits at 9 to 11)
   if (arith == 1) return p.K == 4;

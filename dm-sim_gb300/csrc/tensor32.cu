@@ -7,17 +7,17 @@
 // V's.  Every FP32 operand value is the sum of three BF16 values, each
 // rounded from the remainder of the ones before it (x = h + m + l to 2^-24
 // of |x|; the host split W and V's entries the same way, slices 0..2 of
-// TcDesc).  The six products whose size reaches 2^-16 of the leading one
-// accumulate into three FP32 accumulators in tensor memory -- (h,h); (h,m) and
-// (m,h); (h,l), (m,m) and (l,h) -- which are added in FP32, the small ones
-// first; the three dropped products are below 2^-24 of the leading one.  Each value keeps its own 24-bit precision
+// TcDesc).  The six products whose size reaches 2^-16 of the leading one --
+// (l,h) (m,m) (h,l), then (m,h) (h,m), then (h,h), smallest first --
+// accumulate into one FP32 accumulator in tensor memory; the three dropped
+// ones are below 2^-24 of it.  Each value keeps its own 24-bit precision
 // (no shared exponent per column), so a step's error is FP32 accumulation's,
 // the FP32-pipe passes' own level.
 //
 // Threads, tiles and synchronisation follow tensor64.cu: 512 threads, two
-// blocks per SM (64 registers a thread, 107 KB of shared memory and 256 TMEM
+// blocks per SM (64 registers a thread, 107 KB of shared memory and 64 TMEM
 // columns a block), two independent groups of 8 warps taking alternate tiles,
-// each with its own tile buffer (filled one tile ahead), slice operand, accumulators (3 R TMEM columns), mbarriers and
+// each with its own tile buffer (filled one tile ahead), slice operand, accumulator (R TMEM columns), mbarriers and
 // named barrier.  Per tile:
 //   1. wait for the tile, ket slices -> A;  2. the ket MMAs;  3. ket
 //      accumulator -> FP32 ket outputs in place of the tile;  4. bra slices
@@ -30,9 +30,11 @@
 // DMSIM_ERR_TIMEOUT with rho undefined.
 //
 // What bounds it: issue (60 % active), the ALU and the load/store pipe (40 %
-// each).  A 4-qubit pass at 15 qubits (8.6 GB read and as much written) takes
-// 4.7 ms, 3.7 TB/s; 6.6 ms before the tiles came in by 16-byte copies (5.1) and
-// the orders had accumulators of their own (4.8).
+// each), and the twelve small MMAs of a step, 140 cycles each.  A 4-qubit pass at
+// 15 qubits (8.6 GB read and as much written) takes 4.9 ms, 3.5 TB/s; 6.6 ms before the tiles
+// came in by 16-byte copies.  An accumulator for each order of the slice pairs (six
+// wider MMAs) took 4.7 ms and erred a sixth less, but other roundings than before
+// reach the FP64 diagonals of complex64 states, which are to stay as they were.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -61,11 +63,11 @@ struct T32 {
   static constexpr uint32_t SBO = 16 * R;                  // bytes between 8-row groups of an R-wide operand
   static constexpr uint32_t A_BYTES = 128 * R * 2;         // one slice of the 128 columns
   static constexpr uint32_t B_BYTES = R * R * 2;           // one slice of W or V
-  static constexpr uint32_t SET_COLS = 3 * R;              // the accumulators of one group, an order each
-  static constexpr uint32_t TMEM_COLS = 8 * R;             // two sets, a power of two: 256 (K = 4), 128 (K = 3)
+  static constexpr uint32_t SET_COLS = R;                  // the accumulator of one group
+  static constexpr uint32_t TMEM_COLS = 2 * SET_COLS;      // 64 (K = 4), 32 (K = 3)
   static constexpr uint32_t BUF_BYTES = 2 * ASTR * 4;      // one group's tile buffer
   static_assert(ASTR % 32 == 16 && BUF_BYTES % 16 == 0, "tile buffer layout");
-  static_assert(2 * TMEM_COLS <= 512, "two blocks of two accumulator sets in tensor memory");
+  static_assert(TMEM_COLS <= 512, "two accumulator sets must fit in tensor memory");
 };
 
 // Shared-memory position of local entry e of a loaded tile: 16-entry pieces
@@ -140,37 +142,22 @@ __device__ __forceinline__ void slice_column(const float (&v)[D], int row, int h
   }
 }
 
-// Eight consecutive outputs of this warp's 32 rows: the three orders, the
-// small ones first.
-__device__ __forceinline__ void sum_orders8(uint32_t taddr, uint32_t r, float (&v)[8]) {
-  float o1[8], o2[8];
-  tc::tmem_ld8(taddr, v);
-  tc::tmem_ld8(taddr + r, o1);
-  tc::tmem_ld8(taddr + 2 * r, o2);
-  tc::tmem_wait_ld();
-#pragma unroll
-  for (int c = 0; c < 8; c++) v[c] = __fadd_rn(v[c], __fadd_rn(o1[c], o2[c]));
-}
-
-// One thread issues every product of a step: slice i of the columns against
-// the operator's slices 0..2-i, which are consecutive blocks of one operand, so
-// that the pairs of order i + j meet in the accumulator of order i + j: (0; 0,
-// 1, 2), (1; 0, 1), (2; 0).  Six MMAs of N = 3R, 2R and R instead of twelve of N
-// = R (a small MMA takes about 140 cycles whatever its N), and the leading
-// products (16 bits) keep FP32 accumulators of their own, without the
-// truncation of sums of all orders.
+// One thread issues every product of a step: slice pairs (i of the columns,
+// j of the operator) (2,0) (1,1) (0,2) (1,0) (0,1) (0,0), smallest first,
+// all into the group's one accumulator (N = R).
 template <int K>
 __device__ __forceinline__ void issue_step32(const unsigned char* sA, const unsigned char* sBside, uint32_t dset) {
   using S = T32<K>;
   constexpr int R = S::R;
   const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sBside);
+  constexpr int kPairs[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
 #pragma unroll
-  for (int i = 0; i < kT32Slices; i++) {
+  for (int q = 0; q < 6; q++) {
 #pragma unroll
     for (int kk = 0; kk < R / 16; kk++) {
-      const uint64_t ad = tc::smem_desc(a0 + i * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
-      const uint64_t bd = tc::smem_desc(b0 + kk * 256, tc::kLbo, S::SBO);
-      tc::mma_f16kind(dset + i * R, ad, bd, tc::idesc_bf16_f32(128, (kT32Slices - i) * R), (i == 0 && kk == 0) ? 0u : 1u);
+      const uint64_t ad = tc::smem_desc(a0 + kPairs[q][0] * S::A_BYTES + kk * 256, tc::kLbo, S::SBO);
+      const uint64_t bd = tc::smem_desc(b0 + kPairs[q][1] * S::B_BYTES + kk * 256, tc::kLbo, S::SBO);
+      tc::mma_f16kind(dset, ad, bd, tc::idesc_bf16_f32(128, R), (q == 0 && kk == 0) ? 0u : 1u);
     }
   }
 }
@@ -371,7 +358,8 @@ __global__ void __launch_bounds__(kT32Threads, 2)
 #pragma unroll
       for (int a0 = 0; a0 < D; a0 += 8) {
         float sv[8];
-        sum_orders8(tmem + tlane + half * D + a0, R, sv);
+        tc::tmem_ld8(tmem + tlane + half * D + a0, sv);
+        tc::tmem_wait_ld();
 #pragma unroll
         for (int a = 0; a < 8; a++) buf[yoff(half, a0 + a, r, f)] = sv[a];
       }
@@ -411,7 +399,8 @@ __global__ void __launch_bounds__(kT32Threads, 2)
 #pragma unroll
       for (int b0 = 0; b0 < D; b0 += 8) {
         float sv[8];
-        sum_orders8(tmem + tlane + half * D + b0, R, sv);
+        tc::tmem_ld8(tmem + tlane + half * D + b0, sv);
+        tc::tmem_wait_ld();
         if (tb.allstored) {  // the common case
           float* col = arr + tb.offk[r] + tb.offb[b0];
           const uint64_t s1 = tb.offb[1], s2 = tb.offb[2], s4 = tb.offb[4];
