@@ -86,6 +86,20 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
     nz = s_nz;
     cplx = s_cplx;
   }
+  // simple: real, every output has its own term, outputs 0 and 3 the other's too
+  // (diag: bit 0 for output 0, bit 1 for output 3; not the latter alone) and
+  // outputs 1 and 2 each other's (crossed) or not, and nothing else
+  constexpr uint32_t kOwn = 0x8421u, kCross = 0x0240u;
+  const uint32_t diag = (nz >> 3 & 1) | (nz >> 11 & 2);
+  const bool simple = kSuper && cplx == 0 && (nz & ~(kCross | 0x1008u)) == kOwn && diag != 2 &&
+                      ((nz & kCross) == 0 || (nz & kCross) == kCross);
+  const bool crossed = (nz & kCross) != 0;
+  T sc[kSuper ? 8 : 1];
+  if constexpr (kSuper) {
+    constexpr int at[8] = {0, 3, 12, 15, 5, 6, 9, 10};
+#pragma unroll
+    for (int i = 0; i < 8; i++) sc[i] = s_sr[at[i]];
+  }
   // entry e = a + 2b: which change, which are read (unrolled comparisons,
   // so that the small arrays stay in registers)
   int sidx[4];
@@ -186,6 +200,53 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
         idx[1] = idx[2];
         idx[2] = b;
         idx[3] = a;
+      }
+    } else if (kSuper && simple) {
+      // real terms only between the two diagonal entries and between the two
+      // others (every named channel): 8 to 16 multiply-adds a group, in the order
+      // of the general loop, whose skipped terms cost selects on the FP64 pipe.
+      // 11 qubits, depolarising, half range: 34.7 -> 22.5 us a pass.
+      if (diag == 3) {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const T* x = p ? xi : xr;
+          T* out = p ? outi : outr;
+          out[0] = madd(sc[1], x[3], madd(sc[0], x[0], T(0)));
+          out[3] = madd(sc[3], x[3], madd(sc[2], x[0], T(0)));
+        }
+      } else if (diag == 1) {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const T* x = p ? xi : xr;
+          T* out = p ? outi : outr;
+          out[0] = madd(sc[1], x[3], madd(sc[0], x[0], T(0)));
+          out[3] = madd(sc[3], x[3], T(0));
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const T* x = p ? xi : xr;
+          T* out = p ? outi : outr;
+          out[0] = madd(sc[0], x[0], T(0));
+          out[3] = madd(sc[3], x[3], T(0));
+        }
+      }
+      if (crossed) {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const T* x = p ? xi : xr;
+          T* out = p ? outi : outr;
+          out[2] = madd(sc[5], x[1], madd(sc[4], x[2], T(0)));
+          out[1] = madd(sc[7], x[1], madd(sc[6], x[2], T(0)));
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const T* x = p ? xi : xr;
+          T* out = p ? outi : outr;
+          out[2] = madd(sc[4], x[2], T(0));
+          out[1] = madd(sc[7], x[1], T(0));
+        }
       }
     } else if constexpr (kSuper) {
       // the terms in index order, the zero ones skipped (the same for every thread)
