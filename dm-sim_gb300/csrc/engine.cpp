@@ -291,7 +291,7 @@ HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, const PassSpec& spec, 
     c.fixed_us = 6;
     c.slots = 2.0 * s->sms;
     c.tiles = (double)ntiles;
-    c.tile_us = p.K == 4 ? 10.5 : 6.5;
+    c.tile_us = p.K == 4 ? 8.7 : 5.0;
     return c;
   }
   // picoseconds per entry: memory traffic, or the multiply-adds of the pipe
@@ -339,7 +339,7 @@ size_t plan_half_ranges(dmsim_sim* s, const std::vector<HalfCost>& costs,
                         size_t total) {
   const double state = 2.0 * (double)s->N * (double)esize(s);  // bytes of rho
   const double part = 0.5 * state, full = state;               // a mirror reads and writes a quarter, a half
-  const double us = 1.0 / 5.0e6;                               // at 5 TB/s
+  const double us = 1.0 / 6.2e6;                               // at 6.2 TB/s
   const std::vector<uint32_t> S = plan_half(costs, 3 + part * us, 3 + full * us, &s->half_gain_us);
   std::map<std::pair<uint32_t, std::array<int32_t, 10>>, size_t> maps;
   uint32_t stale = 0;
