@@ -218,8 +218,17 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.herm = s->d_herm;
     if (timed) DM_CUDA(cudaEventRecord(p.ev0, st));
     if (p.stale != p.half) mirror(p.stale, p.half, false);
-    a.pdl = pdl && may_overlap(p.grid);
-    DM_CUDA(launch_pass(a, st));
+    if (!timed && p.merged > 1) {  // one sweep for this pass and the next ones; timed passes run by themselves
+      a.desc = static_cast<const char*>(s->d_desc) + p.multi_off;
+      a.grid = p.multi_grid;
+      a.half = p.half ? reinterpret_cast<const HalfMap*>(static_cast<const char*>(s->d_desc) + p.multi_half_off) : nullptr;
+      a.pdl = pdl && may_overlap(a.grid);
+      DM_CUDA(launch_multi(a, st));
+      i += p.merged - 1;
+    } else {
+      a.pdl = pdl && may_overlap(p.grid);
+      DM_CUDA(launch_pass(a, st));
+    }
     pdl = overlap;
     if (i + 1 == s->passes.size()) mirror(s->end_stale, 0, true);
     if (timed) DM_CUDA(cudaEventRecord(p.ev1, st));
@@ -389,6 +398,114 @@ void capture_passes(dmsim_sim* s) {
   }
 }
 
+// What a pass of a merged run takes, by itself and in the sweep, in the pipe that
+// its multiply-adds load (us): `ops` of them on a thread's 16 entries, 64 cycles
+// each a warp in FP64, fewer in double-float and FP32.  By itself a pass has four
+// times the threads, which small states need.
+struct MergeCost {
+  double apart = 0, pipe = 0, bytes = 0;  // the passes one by one; the sweep's pipe time; their bytes
+};
+void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double frac, MergeCost& c) {
+  double ops = 0;
+  if (op.kind == MO_DENSE) ops = 256;
+  else if (op.kind == MO_REAL) ops = 128;
+  else if (op.kind == MO_HADAMARD) ops = 64;
+  else if (op.kind == MO_CHANNEL) ops = 56;
+  else if (op.kind == MO_MONO)
+    for (int k = 0; k < 4; k++) ops += op.fk[k] == FK_GEN ? 16 : 0;
+  const bool fp64 = s->arith == AR_FP64;
+  const double us = ops * 0.0333 * (fp64 ? 1 : 0.3);
+  const double warps = frac * std::ldexp(1.0, 2 * (int)s->n - 2) / 32 / (4.0 * s->sms);  // of a 1-qubit pass, per scheduler
+  c.apart += 1.8 + std::max(std::max(1.0, warps) * us / 4, p.bytes / 5.8e6);
+  // (FP64 dense operators and channels ran half as fast again in the sweep's few warps)
+  c.pipe += std::max(1.0, warps / 4) * us * (fp64 && (op.kind == MO_DENSE || op.kind == MO_REAL || op.kind == MO_CHANNEL) ? 1.5 : 1);
+  c.bytes += p.bytes;
+}
+
+// Runs of consecutive passes that act on two qubits between them go in one sweep
+// (kernels_multi.cu), their descriptors appended to the blob.  spec_of: the plan
+// entry of each pass, -1 for those that apply no gates.
+size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std::vector<int>& spec_of,
+                    std::vector<unsigned char>& blob, size_t total) {
+  const int n = (int)s->n;
+  const bool had = s->arith == AR_FP64;
+  auto takes = [&](size_t i, int qa, int qb, MultiOp* op) {
+    const PassInfo& p = s->passes[i];
+    if (spec_of[i] < 0 || p.tc || (p.K == 1 && !p.direct1) || p.K > 2) return false;
+    return multi_op(specs[spec_of[i]], qa, qb, had, op);
+  };
+  for (size_t i = 0; i < s->passes.size(); i++) {
+    MultiOp op;
+    int q[2] = {-1, -1};
+    size_t j = i;
+    const uint32_t half = s->passes[i].half;
+    const double frac = half ? 0.5 * (1.0 + std::ldexp(1.0, -std::min(kHalfMaxS, __builtin_popcount(half)))) : 1.0;
+    const double together = frac * 4.0 * (double)s->N * (double)esize(s);
+    MergeCost cost;
+    // the best length so far: a run is cut where a longer one stops paying
+    size_t best = 0;
+    double best_gain = 0, best_bytes = 0;
+    int best_q[2] = {-1, -1};
+    for (; j < s->passes.size() && j - i < (size_t)kMultiOps; j++) {
+      const PassInfo& p = s->passes[j];
+      if (j > i && (p.half != s->passes[i].half || p.stale != p.half)) break;
+      if (!takes(j, -1, -1, &op)) break;
+      const PassSpec& sp = specs[spec_of[j]];
+      int u[4] = {q[0], q[1], -1, -1}, nu = (q[0] >= 0) + (q[1] >= 0);
+      for (int k = 0; k < sp.K; k++)
+        if (sp.q[k] != u[0] && sp.q[k] != u[1] && nu < 4) u[nu++] = sp.q[k];
+      if (nu > 2) break;
+      q[0] = u[0];
+      q[1] = u[1];
+      merge_cost(s, p, op, frac, cost);
+      const double mem = together / 5.5e6;
+      const double gain = 0.9 * cost.apart - (2.0 + std::max(cost.pipe, mem) + 0.3 * std::min(cost.pipe, mem));
+      if (j > i && gain > best_gain) {
+        best = j - i + 1;
+        best_gain = gain;
+        best_bytes = cost.bytes;
+        best_q[0] = q[0];
+        best_q[1] = q[1];
+      }
+    }
+    const size_t count = best;
+    if (count < 2) continue;
+    q[0] = best_q[0];
+    q[1] = best_q[1];
+    if (q[1] < 0)  // one qubit only: any other one that its range's set does not hold
+      for (int c = n - 1; c >= 0 && q[1] < 0; c--)
+        if (c != q[0] && !((s->passes[i].half >> c) & 1)) q[1] = c;
+    if (q[1] < 0) continue;
+    const int qa = std::min(q[0], q[1]), qb = std::max(q[0], q[1]);
+    const size_t off = (total + 255) & ~(size_t)255;
+    blob.resize(std::max(blob.size(), off + sizeof(MultiDesc)));
+    MultiDesc* d = reinterpret_cast<MultiDesc*>(blob.data() + off);
+    std::memset(d, 0, sizeof *d);
+    d->nops = (int)count;
+    d->qa = qa;
+    d->qb = qb;
+    for (size_t k = 0; k < count; k++) takes(i + k, qa, qb, &d->op[k]);
+    total = off + sizeof(MultiDesc);
+    PassInfo& p = s->passes[i];
+    p.merged = (int)count;
+    p.multi_saved = std::max(0.0, best_bytes - together);
+    p.multi_off = off;
+    if (half) {
+      const size_t ho = (total + 15) & ~(size_t)15;
+      blob.resize(std::max(blob.size(), ho + sizeof(HalfMap)));
+      const int32_t hi[4] = {qa, qb, qa + n, qb + n};
+      build_half(n, 0, hi, 4, half, reinterpret_cast<HalfMap*>(blob.data() + ho));
+      p.multi_half_off = ho;
+      total = ho + sizeof(HalfMap);
+    }
+    const uint64_t groups = 1ull << (2 * n - 4);
+    p.multi_grid = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>((groups + kMultiThreads - 1) / kMultiThreads, (uint64_t)s->sms * 12));
+    i += count - 1;
+  }
+  return total;
+}
+
 // Write the descriptors of a plan to the device and capture its launches.
 void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_basic, int arith) {
   ensure_state(s);
@@ -407,6 +524,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
   std::vector<unsigned char> blob(std::max<size_t>(total, 256));
   s->passes.clear();
   std::vector<HalfCost> costs;                // per entry of s->passes
+  std::vector<int> spec_of;                   // its plan entry, -1 if it applies no gates
   std::vector<std::array<int32_t, 10>> geo;   // its L, mhi and high target bits
   const HalfCost whole = {0, 2.5, 0, 1, 1};
   s->keeps_herm = true;
@@ -419,6 +537,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     pi.bytes = conv_bytes;
     s->passes.push_back(pi);
     costs.push_back(whole);
+    spec_of.push_back(-1);
     geo.push_back({});
   }
   for (size_t i = 0; i < specs.size(); i++) {
@@ -431,6 +550,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       pi.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(pi);
       costs.push_back(whole);
+      spec_of.push_back(-1);
       geo.push_back({});
       s->keeps_herm = false;
       continue;
@@ -475,6 +595,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
                             (pi.cls == CLS_MOVE || pi.cls == CLS_SIGNED || pi.cls == CLS_PHASE);
     hc.allowed = tiled_mono ? 0 : half_allowed(hd, specs[i], (int)s->n, pi.direct1);
     costs.push_back(hc);
+    spec_of.push_back((int)i);
     std::array<int32_t, 10> gm = {hd.L, hd.mhi};
     for (int j = 0; j < hd.mhi; j++) gm[2 + j] = hd.hipos[j];
     if (pi.direct1) gm = {0, 2, pi.q0, pi.q0 + (int)s->n};
@@ -488,6 +609,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       rn.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(rn);
       costs.push_back(whole);
+      spec_of.push_back(-1);
       geo.push_back({});
     }
   }
@@ -499,6 +621,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     pi.bytes = conv_bytes;
     s->passes.push_back(pi);
     costs.push_back(whole);
+    spec_of.push_back(-1);
     geo.push_back({});
   }
   // complex64 runs stay whole: their renormalisation averages the two
@@ -507,6 +630,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
   // latency, a half of them no shorter, and the mirrors come on top (9 qubits,
   // 100 layered gates double-float 204 us whole, 253 us half; 10 qubits 376, 330)
   if (s->hermitian && s->keeps_herm && !s->fp32 && s->n >= 10) total = plan_half_ranges(s, costs, geo, blob, total);
+  if (s->n >= 2 && s->direct1) total = merge_passes(s, specs, spec_of, blob, total);
   if (total > 0) {
     DM_CUDA(cudaMalloc(&s->d_desc, total));
     DM_CUDA(cudaMemcpyAsync(s->d_desc, blob.data(), total, cudaMemcpyHostToDevice, s->stream));
@@ -567,7 +691,7 @@ void run(dmsim_sim* s) {
   DM_CUDA(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
   s->last_ms = ms;
   double bytes = 0;
-  for (const PassInfo& p : s->passes) bytes += p.bytes;
+  for (const PassInfo& p : s->passes) bytes += p.bytes - (timed ? 0 : p.multi_saved);
   s->last_bytes = bytes;
   if (timed) {
     s->records.clear();
@@ -1487,7 +1611,7 @@ cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, std::string& err) {
 
 double sim_plan_bytes(dmsim_handle s) {
   double t = 0;
-  for (const PassInfo& p : s->passes) t += p.bytes;
+  for (const PassInfo& p : s->passes) t += p.bytes - p.multi_saved;
   return t;
 }
 

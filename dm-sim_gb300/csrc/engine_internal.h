@@ -25,6 +25,10 @@ struct PassInfo {
   bool real;            // real operator (kernels_real.cu for K <= 2)
   bool direct1;         // 1-qubit pass on the register kernel (kernels_k1.cu)
   bool mono;            // monomial pass on the pipelined kernel (kernels_mono.cu)
+  int merged;           // > 1: launched with the merged - 1 passes after it, in one sweep (kernels_multi.cu)
+  size_t multi_off, multi_half_off;  // its MultiDesc and HalfMap in the device blob
+  unsigned multi_grid;
+  double multi_saved;   // bytes that the sweep moves less than its passes one by one
   int q0;               // first target qubit
   uint32_t half;        // half-range pass: its qubit set S (0: the whole state)
   uint32_t stale;       // the set under which the state is up to date before the pass: a mirror pass goes first

@@ -67,6 +67,8 @@ cudaError_t launch_pass1(const LaunchArgs& a, cudaStream_t s);
 // grid, 0 for a pass that it does not take, and the launch.
 unsigned mono_grid(int K, int cls, int tile_entries, uint64_t ntiles, int sms);
 cudaError_t launch_mono(const LaunchArgs& a, cudaStream_t s);
+// Several narrow passes in one sweep (kernels_multi.cu): desc is a MultiDesc.
+cudaError_t launch_multi(const LaunchArgs& a, cudaStream_t s);
 // Real-operator instances of the 1- and 2-qubit DENSE/SPARSE kernels (kernels_real.cu).
 cudaError_t launch_pass_real(const LaunchArgs& a, cudaStream_t s);
 // Tensor-core passes (tensor.cu): launch, and resident blocks per SM.

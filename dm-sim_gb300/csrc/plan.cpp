@@ -780,6 +780,73 @@ uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uin
   return build_tc_k<4>(p, n, static_cast<TcDesc<4>*>(out), f, ntiles, tile_entries, slices, per_entry);
 }
 
+// ---------------------------------------------------------------- several passes in one sweep
+bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
+  if (p.transpose || p.rlin || p.ket_only || p.K < 1 || p.K > 2) return false;
+  std::memset(out, 0, sizeof *out);
+  if (p.K == 2) {
+    // CX alone: U swaps the target where the control is 1
+    if (p.cls != CLS_MOVE) return false;
+    for (int c = 0; c < 2; c++) {
+      bool cx = true;
+      for (int r = 0; r < 4; r++) {
+        const int s = (r >> c) & 1 ? r ^ (2 >> c) : r;
+        cx = cx && p.U[r * 4 + s] == cplx(1, 0);
+      }
+      if (!cx) continue;
+      out->kind = MO_CX;
+      out->p = p.q[c] == qa ? 0 : 1;
+      return true;
+    }
+    return false;
+  }
+  out->p = p.q[0] == qa ? 0 : 1;
+  if (p.super) {
+    // the register kernel's simple channels
+    uint32_t nz = 0;
+    for (int i = 0; i < 16; i++) {
+      if (p.U[i].imag() != 0) return false;
+      if (p.U[i].real() != 0) nz |= 1u << i;
+    }
+    const uint32_t diag = (nz >> 3 & 1) | (nz >> 11 & 2), cross = nz & 0x0240u;
+    if ((nz & ~(0x0240u | 0x1008u)) != 0x8421u || diag == 2 || (cross && cross != 0x0240u)) return false;
+    static const int at[8] = {0, 3, 12, 15, 5, 6, 9, 10};
+    for (int i = 0; i < 8; i++) out->c[i] = p.U[at[i]].real();
+    out->kind = MO_CHANNEL;
+    out->flags = (int)diag | (cross ? 4 : 0);
+    return true;
+  }
+  std::unique_ptr<PassDesc<1>> d(new PassDesc<1>);
+  build_k<1>(p, 17, d.get(), nullptr, nullptr, nullptr, 8);  // factors, kinds and flags: the same for every size
+  const PassOp<1>& op = d->op;
+  if (p.cls == CLS_DENSE || p.cls == CLS_SPARSE) {
+    if (p.cls == CLS_SPARSE) return false;
+    if (hadamard && (d->h.flags & kPassHadamard)) {
+      out->kind = MO_HADAMARD;
+      out->flags = (op.ure[0] * op.ure[1] < 0 ? 1 : 0) | (op.ure[0] * op.ure[2] < 0 ? 2 : 0);
+      return true;
+    }
+    out->kind = d->h.flags & kPassRealOperator ? MO_REAL : MO_DENSE;
+    for (int i = 0; i < 4; i++) {
+      out->c[i] = op.ure[i];
+      out->c[4 + i] = op.uim[i];
+      out->c[8 + i] = op.vre[i];
+      out->c[12 + i] = op.vim[i];
+    }
+    return true;
+  }
+  if (op.src[0] != op.srcb[0] || op.src[1] != op.srcb[1]) return false;
+  out->kind = MO_MONO;
+  out->flags = op.src[0] == 1 ? 1 : 0;
+  for (int i = 0; i < 4; i++) {
+    out->c[i] = op.fre[i];
+    out->c[4 + i] = op.fim[i];
+    out->fk[i] = op.fk[i];
+    if (op.fk[i] != FK_ONE) out->flags |= 2;
+  }
+  return true;
+}
+
 // ---------------------------------------------------------------- half-range passes
 uint32_t half_allowed(const PassHeader& h, const PassSpec& p, int n, bool direct1) {
   if (p.transpose || p.rlin || p.ket_only) return 0;
