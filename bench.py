@@ -562,7 +562,7 @@ def main():
                        "basic_gates": nbasic,
                        "l2": "inputs larger than L2 (rho = %.1f GB)" % (16.0 * N / 1e9), "parallelism": "replicas"},
             "state": "FP64 rho in and out; fused passes at FP64 width: 3/4-qubit operators on the tensor cores "
-                     "with 7 BF16 digits per operand, exact integer order sums and one rounding to FP64 per output "
+                     "with 7 FP16 digits per operand, exact integer order sums and one rounding to FP64 per output "
                      "(55-bit significands per column), other passes in FP64; plain = the reference's method in FP64",
             "plain_s": plain_s, "plain_passes": plain_passes, "plain_kernels": plain_kernels,
             "speedup_fused_vs_plain": (plain_s / value) if plain_s else None,
