@@ -410,13 +410,14 @@ void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double
   if (op.kind == MO_DENSE) ops = 256;
   else if (op.kind == MO_REAL) ops = 128;
   else if (op.kind == MO_HADAMARD) ops = 64;
-  else if (op.kind == MO_CHANNEL) ops = 56;
+  else if (op.kind == MO_CHANNEL || op.kind == MO_CHANNEL2) ops = 56;
   else if (op.kind == MO_MONO)
     for (int k = 0; k < 4; k++) ops += op.fk[k] == FK_GEN ? 16 : 0;
   const bool fp64 = s->arith == AR_FP64;
   const double us = ops * 0.0333 * (fp64 ? 1 : 0.3);
   const double warps = frac * std::ldexp(1.0, 2 * (int)s->n - 2) / 32 / (4.0 * s->sms);  // of a 1-qubit pass, per scheduler
-  c.apart += 1.8 + std::max(std::max(1.0, warps) * us / 4, p.bytes / 5.8e6);
+  // (a 2-qubit channel's tiles take twice their pipe's time by themselves)
+  c.apart += 1.8 + std::max(std::max(1.0, warps) * us / (op.kind == MO_CHANNEL2 ? 2 : 4), p.bytes / 5.8e6);
   // (FP64 dense operators and channels ran half as fast again in the sweep's few warps)
   c.pipe += std::max(1.0, warps / 4) * us * (fp64 && (op.kind == MO_DENSE || op.kind == MO_REAL || op.kind == MO_CHANNEL) ? 1.5 : 1);
   c.bytes += p.bytes;

@@ -39,7 +39,7 @@ __device__ __forceinline__ df64 m_sub(df64 a, df64 b) { return a + -b; }
 
 template <typename T>
 struct OpShared {
-  T c[16];
+  T c[32];
   int kind, p, flags;
   int8_t fk[4];
 };
@@ -212,6 +212,26 @@ __device__ __forceinline__ void apply_cx(T (&x)[16]) {
   for (int ket = 0; ket < 4; ket++) swap2(x[ket + 4 * c], x[ket + 4 * (c + t)]);
 }
 
+// A 2-qubit channel of real terms between the diagonal entries and of every other
+// entry's own, first qubit F of the pair: index i's bits are at entry bits F, 1 - F.
+template <typename T, int F>
+__device__ __forceinline__ void apply_channel2(const OpShared<T>& op, T (&x)[16]) {
+  constexpr int b0 = 1 << F, b1 = 2 >> F;
+  auto at = [](int a, int b) { return ((a & 1) * b0 + (a >> 1) * b1) + 4 * ((b & 1) * b0 + (b >> 1) * b1); };
+  T y[4];
+#pragma unroll
+  for (int o = 0; o < 4; o++) {
+    T acc = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc = madd(op.c[o * 4 + j], x[at(j, j)], acc);
+    y[o] = acc;
+  }
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) x[at(a, b)] = a == b ? y[a] : madd(op.c[16 + a * 4 + b], x[at(a, b)], T(0));
+}
+
 template <typename T, bool HALF>
 __global__ void __launch_bounds__(kMultiThreads, 3) k_multi(T* __restrict__ re, T* __restrict__ im,
                                                             const MultiDesc* __restrict__ dp, int n,
@@ -219,7 +239,7 @@ __global__ void __launch_bounds__(kMultiThreads, 3) k_multi(T* __restrict__ re, 
                                                             const int* __restrict__ herm) {
   __shared__ OpShared<T> s_op[kMultiOps];
   const int nops = dp->nops;
-  for (int i = threadIdx.x; i < nops * 16; i += blockDim.x) s_op[i >> 4].c[i & 15] = coef<T>(dp->op[i >> 4].c[i & 15]);
+  for (int i = threadIdx.x; i < nops * 32; i += blockDim.x) s_op[i >> 5].c[i & 31] = coef<T>(dp->op[i >> 5].c[i & 31]);
   for (int i = threadIdx.x; i < nops; i += blockDim.x) {
     s_op[i].kind = dp->op[i].kind;
     s_op[i].p = dp->op[i].p;
@@ -259,6 +279,14 @@ __global__ void __launch_bounds__(kMultiThreads, 3) k_multi(T* __restrict__ re, 
         } else {
           apply_cx<T, 1>(xr);
           apply_cx<T, 1>(xi);
+        }
+      } else if (op.kind == MO_CHANNEL2) {
+        if (op.p == 0) {
+          apply_channel2<T, 0>(op, xr);
+          apply_channel2<T, 0>(op, xi);
+        } else {
+          apply_channel2<T, 1>(op, xr);
+          apply_channel2<T, 1>(op, xi);
         }
       } else if (op.p == 0) {
         apply1<T, 0>(op, xr, xi);

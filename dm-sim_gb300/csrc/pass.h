@@ -99,12 +99,13 @@ struct PassDesc {
 
 // ---- several narrow passes in one sweep (kernels_multi.cu)
 constexpr int kMultiOps = 16, kMultiThreads = 128;
-enum MultiKind : int32_t { MO_DENSE = 0, MO_REAL = 1, MO_HADAMARD = 2, MO_MONO = 3, MO_CHANNEL = 4, MO_CX = 5 };
+enum MultiKind : int32_t { MO_DENSE = 0, MO_REAL = 1, MO_HADAMARD = 2, MO_MONO = 3, MO_CHANNEL = 4, MO_CX = 5, MO_CHANNEL2 = 6 };
 struct MultiOp {
-  // DENSE, REAL: U, V (re, im each); MONO: f re, im at [a * 2 + b]; CHANNEL: its eight terms
-  double c[16];
+  // DENSE, REAL: U, V (re, im each); MONO: f re, im at [a * 2 + b]; CHANNEL: its eight terms;
+  // CHANNEL2: the terms between the diagonal entries at [to * 4 + from], then the others' own at 16 + [a * 4 + b]
+  double c[32];
   int32_t kind;
-  int32_t p;      // 0: on qubit qa (CX: its control), 1: on qubit qb
+  int32_t p;      // 0: on qubit qa (CX: its control; CHANNEL2: its first qubit), 1: on qubit qb
   int32_t flags;  // HADAMARD: 1 outputs swapped, 2 the mixed ones negated; MONO: 1 X, 2 factors; CHANNEL: as its kernel
   int8_t fk[4];   // MONO: FactorKind at [a * 2 + b]
 };

@@ -784,6 +784,20 @@ uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uin
 bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
   if (p.transpose || p.rlin || p.ket_only || p.K < 1 || p.K > 2) return false;
   std::memset(out, 0, sizeof *out);
+  if (p.K == 2 && p.super) {
+    // depolarising and its like: between the diagonal entries all terms, elsewhere an entry's own
+    for (int o = 0; o < 16; o++)
+      for (int j = 0; j < 16; j++) {
+        const cplx m = p.U[o * 16 + j];
+        const bool od = o / 4 == o % 4, jd = j / 4 == j % 4;
+        const bool term = od ? jd : o == j;
+        if (m.imag() != 0 || (m.real() != 0) != term) return false;
+        if (term) out->c[od ? (o / 4) * 4 + j / 4 : 16 + o] = m.real();
+      }
+    out->kind = MO_CHANNEL2;
+    out->p = p.q[0] == qa ? 0 : 1;
+    return true;
+  }
   if (p.K == 2) {
     // CX alone: U swaps the target where the control is 1
     if (p.cls != CLS_MOVE) return false;

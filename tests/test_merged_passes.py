@@ -21,6 +21,8 @@ def program(n, rng, noise):
             if x < 0.35:
                 c, t = pair if rng.random() < 0.5 else pair[::-1]
                 out.append((OP["CX"], (c, t), 0.0, 0.0, 0.0))
+            elif x < 0.42 and noise:
+                out.append(("depolarizing2", tuple(pair if rng.random() < 0.5 else pair[::-1]), float(rng.uniform(0.01, 0.4))))
             elif x < 0.5 and noise:
                 kind = str(rng.choice(["depolarizing", "amplitude_damping", "phase_damping", "bit_flip", "phase_flip"]))
                 out.append((kind, (pair[int(rng.integers(2))],), float(rng.uniform(0.01, 0.4))))
