@@ -19,23 +19,12 @@ namespace dmg {
 
 namespace {
 
-// x / 2: one off the exponent field, on the ALU, where that is exact; zeros are
-// themselves.
-__device__ __forceinline__ double half_of(double x) {
-  const int h = __double2hiint(x), l = __double2loint(x);
-  const uint32_t e = (uint32_t)h & 0x7FF00000u;
-  if (e == 0x00100000u || e == 0x7FF00000u || (e == 0 && ((h << 1) | l))) return 0.5 * x;
-  return __hiloint2double(h - (e ? 0x00100000 : 0), l);
-}
 // -x if n (32-bit integer work: a select of doubles takes the FP64 pipe)
 __device__ __forceinline__ double xor_sign(double x, bool n) {
   return __hiloint2double(__double2hiint(x) ^ (n ? (int)0x80000000 : 0), __double2loint(x));
 }
 __device__ __forceinline__ float xor_sign(float x, bool n) { return n ? -x : x; }
 __device__ __forceinline__ df64 xor_sign(df64 x, bool n) { return n ? -x : x; }
-__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
-__device__ __forceinline__ df64 half_of(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
-__device__ __forceinline__ df64 operator-(df64 a, df64 b) { return a + -b; }
 
 template <typename T, int CLS_, bool HALF>
 __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict__ im,

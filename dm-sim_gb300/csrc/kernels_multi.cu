@@ -25,18 +25,6 @@ namespace dmg {
 
 namespace {
 
-__device__ __forceinline__ double m_half(double x) {
-  const int h = __double2hiint(x), l = __double2loint(x);
-  const uint32_t e = (uint32_t)h & 0x7FF00000u;
-  if (e == 0x00100000u || e == 0x7FF00000u || (e == 0 && ((h << 1) | l))) return 0.5 * x;
-  return __hiloint2double(h - (e ? 0x00100000 : 0), l);
-}
-__device__ __forceinline__ float m_half(float x) { return 0.5f * x; }
-__device__ __forceinline__ df64 m_half(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
-__device__ __forceinline__ double m_sub(double a, double b) { return a - b; }
-__device__ __forceinline__ float m_sub(float a, float b) { return a - b; }
-__device__ __forceinline__ df64 m_sub(df64 a, df64 b) { return a + -b; }
-
 template <typename T>
 struct OpShared {
   T c[32];
@@ -140,11 +128,11 @@ __device__ __forceinline__ void apply1(const OpShared<T>& op, T (&xr)[16], T (&x
   } else if (kind == MO_HADAMARD) {
     each_group<T, P>(xr, xi, [&](T& r0, T& r1, T& r2, T& r3, T& i0, T& i1, T& i2, T& i3) {
       auto h = [](T& x0, T& x1, T& x2, T& x3) {
-        const T s0 = x0 + x1, d0 = m_sub(x0, x1), s1 = x2 + x3, d1 = m_sub(x2, x3);
-        x0 = m_half(s0 + s1);
-        x1 = m_half(d0 + d1);
-        x2 = m_half(m_sub(s0, s1));
-        x3 = m_half(m_sub(d0, d1));
+        const T s0 = x0 + x1, d0 = x0 - x1, s1 = x2 + x3, d1 = x2 - x3;
+        x0 = half_of(s0 + s1);
+        x1 = half_of(d0 + d1);
+        x2 = half_of(s0 - s1);
+        x3 = half_of(d0 - d1);
       };
       h(r0, r1, r2, r3);
       h(i0, i1, i2, i3);

@@ -53,6 +53,7 @@ __device__ __forceinline__ df64 operator+(df64 a, df64 b) {
   const df64 s = two_sum(a.hi, b.hi);
   return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
 }
+__device__ __forceinline__ df64 operator-(df64 a, df64 b) { return a + -b; }
 __device__ __forceinline__ df64 operator*(df64 a, df64 b) {
   const float p = __fmul_rn(a.hi, b.hi);
   float e = __fmaf_rn(a.hi, b.hi, -p);
@@ -160,6 +161,17 @@ __device__ __forceinline__ double flip(double x) {
 }
 __device__ __forceinline__ float flip(float x) { return __int_as_float(__float_as_int(x) ^ (int)0x80000000); }
 __device__ __forceinline__ df64 flip(df64 x) { return df64(flip(x.hi), flip(x.lo)); }
+
+// x / 2: one off the exponent field, on the ALU, where that is exact; zeros are
+// themselves.
+__device__ __forceinline__ double half_of(double x) {
+  const int h = __double2hiint(x), l = __double2loint(x);
+  const uint32_t e = (uint32_t)h & 0x7FF00000u;
+  if (e == 0x00100000u || e == 0x7FF00000u || (e == 0 && ((h << 1) | l))) return 0.5 * x;
+  return __hiloint2double(h - (e ? 0x00100000 : 0), l);
+}
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+__device__ __forceinline__ df64 half_of(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
 
 template <int K>
 __device__ __forceinline__ int pext_local(int loc, const int* lpos) {
