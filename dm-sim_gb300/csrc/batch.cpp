@@ -255,7 +255,9 @@ void build(dmsim_batch* b) {
   cudaGraph_t graph = nullptr;
   std::string werr;
   B_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = cudaEventRecord(b->fork, b->stream);
+  // the error word starts at 0 before either branch (a batch may have no queue)
+  cudaError_t e = cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream);
+  if (e == cudaSuccess) e = cudaEventRecord(b->fork, b->stream);
   std::vector<char> used(b->side.size(), 0);
   int k = 0;
   for (int c = 0; c < nc && e == cudaSuccess; c++) {

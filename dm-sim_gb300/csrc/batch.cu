@@ -236,7 +236,6 @@ static cudaError_t launch_t(const BatchLaunch& a, cudaStream_t s) {
   k_batch_init<T><<<(a.ncirc + 255) / 256, 256, 0, s>>>(re, a.circs, a.ncirc);
   e = cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(a.done, 0, (size_t)a.nranges * sizeof(unsigned), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.err, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   k_batch<T><<<a.grid, kThreads, smem, s>>>(re, im, a.blob, a.ranges, a.nranges, a.nitems, a.next, a.done, a.err,
                                             a.spin_limit);
