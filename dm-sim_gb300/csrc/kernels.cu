@@ -84,20 +84,23 @@ cudaError_t launch_pass(const LaunchArgs& a, cudaStream_t s) {
 }
 
 template <typename T, int K, int CLS>
-static int occ_query() {
+static cudaError_t occ_query(int* blocks) {
   constexpr int D = 1 << K;
   int nb = 0;
   const size_t smem = pass_smem_bytes<T, K, CLS>(kThreads * D);
-  if (configure_pass<T, K, CLS, false>() != cudaSuccess) return 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pass<T, K, CLS, false>, kThreads, smem) != cudaSuccess) return 1;
-  return nb > 0 ? nb : 1;
+  cudaError_t e = configure_pass<T, K, CLS, false>();
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pass<T, K, CLS, false>, kThreads, smem);
+  *blocks = nb > 0 ? nb : 1;
+  return e;
 }
-// Asked once per instance and process: an upload asks for every pass, and the
+// Asked once per instance and context: an upload asks for every pass, and the
 // attribute calls and the query took 6 us each time.
 template <typename T, int K, int CLS>
 static int occ_one() {
-  static const int nb = occ_query<T, K, CLS>();
-  return nb;
+  static PerContext occ;
+  int nb = 1;
+  return occ.get(occ_query<T, K, CLS>, &nb) == cudaSuccess ? nb : 1;
 }
 
 template <typename T, int K>

@@ -21,6 +21,7 @@
 
 #include "kernels.h"
 #include "pass_device.cuh"
+#include "per_context.h"
 #include "tc.cuh"
 
 namespace dmg {
@@ -180,15 +181,15 @@ template <typename T, int K, int CLS>
 cudaError_t launch_mono_one(const LaunchArgs& a, cudaStream_t s) {
   using M = Mono<T, K>;
   constexpr int smem = M::ST * M::STAGE;
-  static int configured = 0;  // per instance; attribute set once per process
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(k_mono<T, K, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_mono<T, K, CLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  static PerContext configured;  // per instance
+  const cudaError_t e = configured.get([](int*) {
+    cudaError_t c = cudaFuncSetAttribute(k_mono<T, K, CLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (c == cudaSuccess)
+      c = cudaFuncSetAttribute(k_mono<T, K, CLS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    configured = 1;
-  }
+    return c;
+  });
+  if (e != cudaSuccess) return e;
   return launch_kernel(a.pdl, k_mono<T, K, CLS>, a.grid, M::NT, smem, s, static_cast<T*>(a.re), static_cast<T*>(a.im),
                        static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
 }

@@ -9,6 +9,7 @@
 #include "kernels.h"
 #include "pass.h"
 #include "pass_device.cuh"
+#include "per_context.h"
 
 namespace dmg {
 
@@ -92,12 +93,9 @@ inline cudaError_t launch_one(const LaunchArgs& a, cudaStream_t s) {
     }
   }
   const size_t smem = pass_smem_bytes<T, K, CLS>(a.tile_entries);
-  static int configured = 0;  // per instance; attribute set once per process
-  if (!configured) {
-    cudaError_t e = configure_pass<T, K, CLS, HALF>();
-    if (e != cudaSuccess) return e;
-    configured = 1;
-  }
+  static PerContext configured;  // per instance
+  const cudaError_t e = configured.get([](int*) { return configure_pass<T, K, CLS, HALF>(); });
+  if (e != cudaSuccess) return e;
   return launch_kernel(a.pdl, k_pass<T, K, CLS, HALF>, a.grid, kThreads, smem, s, static_cast<T*>(a.re),
                        static_cast<T*>(a.im), static_cast<const PassDesc<K>*>(a.desc), a.half, a.herm);
 }

@@ -31,6 +31,7 @@
 
 #include "kernels.h"
 #include "pass_device.cuh"
+#include "per_context.h"
 #include "tc.cuh"
 
 namespace dmg {
@@ -462,12 +463,9 @@ static cudaError_t configure_tc() {
 template <int K, typename T>
 static cudaError_t launch_tc_k(const LaunchArgs& a, cudaStream_t s) {
   constexpr size_t smem = tc_smem_bytes<K, T>();
-  static int configured = 0;
-  if (!configured) {
-    cudaError_t e = configure_tc<K, T>();
-    if (e != cudaSuccess) return e;
-    configured = 1;
-  }
+  static PerContext configured;
+  const cudaError_t e = configured.get([](int*) { return configure_tc<K, T>(); });
+  if (e != cudaSuccess) return e;
   return launch_kernel(a.pdl, k_pass_tc<K, T>, a.grid, kThreads, smem, s, static_cast<T*>(a.re), static_cast<T*>(a.im),
                        static_cast<const TcDesc<K>*>(a.desc), a.err, a.half, a.herm);
 }
@@ -483,16 +481,17 @@ cudaError_t launch_pass_tc(const LaunchArgs& a, cudaStream_t s) {
 // 512 TMEM columns.  (The runtime occupancy query reported one block for
 // this kernel although two fit; the launch statistics confirm two.)
 template <int K, typename T>
-static int tc_occ() {
+static cudaError_t tc_occ_query(int* blocks) {
   constexpr size_t smem = tc_smem_bytes<K, T>();
-  if (configure_tc<K, T>() != cudaSuccess) return 1;
   cudaFuncAttributes fa;
   int dev = 0, smem_sm = 0, regs_sm = 0, threads_sm = 0;
-  if (cudaFuncGetAttributes(&fa, k_pass_tc<K, T>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev) != cudaSuccess)
-    return 1;
+  cudaError_t e = configure_tc<K, T>();
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_pass_tc<K, T>);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&threads_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev);
+  if (e != cudaSuccess) return e;
   const int by_smem = smem_sm / (int)(smem + fa.sharedSizeBytes + 1024);
   const int by_regs = regs_sm / (fa.numRegs * kThreads);
   const int by_threads = threads_sm / kThreads;
@@ -501,14 +500,20 @@ static int tc_occ() {
   nb = nb < by_regs ? nb : by_regs;
   nb = nb < by_threads ? nb : by_threads;
   nb = nb < by_tmem ? nb : by_tmem;
-  return nb > 0 ? nb : 1;
+  *blocks = nb > 0 ? nb : 1;
+  return cudaSuccess;
+}
+template <int K, typename T>
+static int tc_occ() {
+  static PerContext occ;
+  int nb = 1;
+  return occ.get(tc_occ_query<K, T>, &nb) == cudaSuccess ? nb : 1;
 }
 
 int tc_blocks_per_sm(int K, int arith) {
   if (arith == AR_FP64) return 1;  // the FP64-width kernel: one persistent block per SM (tensor64.cu)
   if (arith == AR_FP32) return 2;  // the complex64 kernel: two persistent blocks per SM (tensor32.cu)
-  static const int nb[2] = {tc_occ<3, df64>(), tc_occ<4, df64>()};  // asked once per process
-  return nb[K == 3 ? 0 : 1];
+  return K == 3 ? tc_occ<3, df64>() : tc_occ<4, df64>();
 }
 
 }  // namespace dmg

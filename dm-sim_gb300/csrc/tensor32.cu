@@ -41,6 +41,7 @@
 
 #include "kernels.h"
 #include "pass.h"
+#include "per_context.h"
 #include "tc.cuh"
 
 namespace dmg {
@@ -447,12 +448,9 @@ static cudaError_t configure_tc32() {
 
 template <int K>
 static cudaError_t launch_tc32_k(const LaunchArgs& a, cudaStream_t s) {
-  static int configured = 0;
-  if (!configured) {
-    cudaError_t e = configure_tc32<K>();
-    if (e != cudaSuccess) return e;
-    configured = 1;
-  }
+  static PerContext configured;
+  const cudaError_t e = configured.get([](int*) { return configure_tc32<K>(); });
+  if (e != cudaSuccess) return e;
   return launch_kernel(a.pdl, k_pass_tc32<K>, a.grid, kT32Threads, t32_smem_bytes<K>(), s, static_cast<float*>(a.re),
                        static_cast<float*>(a.im), static_cast<const TcDesc<K>*>(a.desc), a.err);
 }

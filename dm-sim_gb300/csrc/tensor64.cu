@@ -63,6 +63,7 @@
 
 #include "kernels.h"
 #include "pass_device.cuh"
+#include "per_context.h"
 #include "tc.cuh"
 
 namespace dmg {
@@ -674,12 +675,9 @@ static cudaError_t configure_tc64() {
 
 template <int K>
 static cudaError_t launch_tc64_k(const LaunchArgs& a, cudaStream_t s) {
-  static int configured = 0;
-  if (!configured) {
-    cudaError_t e = configure_tc64<K>();
-    if (e != cudaSuccess) return e;
-    configured = 1;
-  }
+  static PerContext configured;
+  const cudaError_t e = configured.get([](int*) { return configure_tc64<K>(); });
+  if (e != cudaSuccess) return e;
   return launch_kernel(a.pdl, k_pass_tc64<K>, a.grid, kT64Threads, t64_smem_bytes<K>(), s, static_cast<uint64_t*>(a.re),
                        static_cast<uint64_t*>(a.im), static_cast<const TcDesc64<K>*>(a.desc), a.err, a.half, a.herm,
                        a.n);
