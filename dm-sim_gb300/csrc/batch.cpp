@@ -51,7 +51,7 @@ struct dmsim_batch {
   BatchRange* d_ranges = nullptr;
   unsigned long long* d_next = nullptr;
   unsigned* d_done = nullptr;
-  int* d_err = nullptr;
+  int* d_err = nullptr;                // set by an expired wait of the queue or of a wide circuit's tensor pass
   int nranges = 0;
   unsigned long long nitems = 0;
   unsigned grid = 0;
@@ -270,7 +270,7 @@ void build(dmsim_batch* b) {
     }
     void *re = nullptr, *im = nullptr;
     if (e == cudaSuccess) e = dmsim_device_state(b->sims[c], &re, &im) == DMSIM_OK ? cudaSuccess : cudaErrorUnknown;
-    if (e == cudaSuccess) e = sim_enqueue(b->sims[c], st, werr);
+    if (e == cudaSuccess) e = sim_enqueue(b->sims[c], st, b->d_err, werr);
     if (e == cudaSuccess)
       e = launch_circuit_epilogue(static_cast<const double*>(re), (int)b->nq[c], b->d_diag + b->circs[c].diag_off,
                                   b->d_zz + b->circs[c].zz_off, st);
@@ -486,11 +486,6 @@ int dmsim_batch_run(dmsim_batch_handle b) {
     b->last_ms = ms;
     int err = 0;
     B_CUDA(cudaMemcpy(&err, b->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    for (dmsim_handle h : b->sims) {  // a wide circuit's tensor pass whose bounded wait ran out
-      int f = 0;
-      if (h) B_CUDA(sim_take_error(h, &f));
-      err |= f;
-    }
     if (err) {
       // Work after the expired wait ran on partly updated states: make every
       // output NaN (all-ones bytes) rather than leave plausible values behind.

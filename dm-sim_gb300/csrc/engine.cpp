@@ -151,10 +151,11 @@ void check_qubits(const dmsim_sim* s, const GateRec& g) {
       if (g.qb[i] == g.qb[j]) throw DmError{DMSIM_ERR_ARG, "a gate's qubits must be distinct"};
 }
 
-// Launch the planned passes on stream st (captured or direct).  A timed pass
+// Launch the planned passes on stream st (captured or direct); a wait that runs
+// out sets *err_word.  A timed pass
 // includes the mirror pass that it needs before it, the last one the mirror
 // that brings the whole state up to date.
-void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
+void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
   // Whether the next kernel may start under the one before it (kernels.h), so
   // that launch, tables and tensor-memory allocation overlap: states up to 12
   // qubits (5 qubits gate by gate 1870 -> 1380 us, 8 qubits fused 565 -> 415, 12
@@ -209,7 +210,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st) {
     a.tc = p.tc;
     a.real = p.real;
     a.hadamard = p.hadamard;
-    a.err = s->d_err;
+    a.err = err_word;
     a.direct1 = p.direct1;
     a.mono = p.mono;
     a.q0 = p.q0;
@@ -383,7 +384,7 @@ void capture_passes(dmsim_sim* s) {
   cudaGraph_t graph = nullptr;
   DM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   try {
-    enqueue_passes(s, false, s->stream);
+    enqueue_passes(s, false, s->stream, s->d_err);
   } catch (...) {
     cudaStreamEndCapture(s->stream, &graph);
     if (graph) cudaGraphDestroy(graph);
@@ -672,7 +673,7 @@ void run(dmsim_sim* s) {
     }
   }
   DM_CUDA(cudaEventRecord(s->ev0, s->stream));
-  if (timed || !s->gexec) enqueue_passes(s, timed, s->stream);
+  if (timed || !s->gexec) enqueue_passes(s, timed, s->stream, s->d_err);
   else DM_CUDA(cudaGraphLaunch(s->gexec, s->stream));
   DM_CUDA(cudaEventRecord(s->ev1, s->stream));
   DM_CUDA(cudaEventSynchronize(s->ev1));
@@ -1595,14 +1596,14 @@ int sim_upload_plan(dmsim_handle h, const std::vector<PassSpec>& specs, uint32_t
   });
 }
 
-cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, std::string& err) {
+cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, int* err_word, std::string& err) {
   if (!s || !s->uploaded) {
     err = "sim_enqueue: no uploaded plan";
     return cudaErrorInvalidValue;
   }
   try {
     DM_CUDA(launch_set_zero_state(s->d_re, s->d_im, s->N, s->fp32, st));
-    enqueue_passes(s, false, st);
+    enqueue_passes(s, false, st, err_word);
   } catch (const DmError& e) {
     err = e.msg;
     return cudaErrorUnknown;
@@ -1614,14 +1615,6 @@ double sim_plan_bytes(dmsim_handle s) {
   double t = 0;
   for (const PassInfo& p : s->passes) t += p.bytes - p.multi_saved;
   return t;
-}
-
-cudaError_t sim_take_error(dmsim_handle s, int* flag) {
-  int h = 0;
-  cudaError_t e = cudaMemcpy(&h, s->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && h) e = cudaMemset(s->d_err, 0, sizeof(int));
-  *flag = h;
-  return e;
 }
 
 }  // namespace dmg

@@ -49,11 +49,10 @@ struct PassRecord {
 
 // For the batched sweep (batch.cpp): upload a plan made elsewhere (no real-linear
 // gates, no channels); enqueue |0..0><0..0| and every pass of
-// s's uploaded plan on stream st (e.g. inside another stream's capture), and
-// read-and-clear s's device error flag (set by an expired bounded wait).
+// s's uploaded plan on stream st (e.g. inside another stream's capture); a bounded
+// wait that runs out sets the caller's device word *err_word.
 int sim_upload_plan(dmsim_handle s, const std::vector<PassSpec>& specs, uint32_t n_basic);
-cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, std::string& err);
-cudaError_t sim_take_error(dmsim_handle s, int* flag);
+cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, int* err_word, std::string& err);
 // algorithmic bytes of s's uploaded plan (reads + writes of every pass)
 double sim_plan_bytes(dmsim_handle s);
 
