@@ -295,20 +295,22 @@ void build(dmsim_batch* b) {
   }
 }
 
-// From how many qubits on a circuit is a wide one.  A circuit of the 4-layer
-// ansatz takes, among many (wide, work queue): 6 qubits 10.3 and 2.6 us, 7 qubits
-// 11 and 12, 8 qubits 17 and 65, 9 qubits 77 and 311 -- and the queue's chain of
-// passes 0.45 ms at 6 qubits, so a few 6-qubit circuits are better off wide too (8
-// of them 0.09 and 0.45 ms).  More of them would be up to 64 (0.60 and 0.71 ms), but
-// a wide circuit also costs 0.3 ms more to upload.  Gate by gate, 32 circuits: 6
-// qubits 0.77 ms wide, 0.34 in the queue, 7 qubits 0.94 and 1.38; double-float: 7
-// qubits 0.41 and 0.30, 8 qubits 0.41 and 0.56.
+// From how many qubits on a circuit is a wide one.  A wide circuit runs faster but
+// costs 0.3 to 0.5 ms more to upload and close (a handle, its copies, a graph node
+// per pass), so the line lies where it pays for that within about ten runs, by the
+// host's clock around upload(), run() and close().  4-layer ansatz, all of one size,
+// milliseconds a run (queue, wide) and the runs to pay: 6 qubits, 8 circuits 0.47,
+// 0.10, 4; 32: 0.59, 0.27, 19.  7 qubits, 8: 0.83, 0.10, 2; 32: 1.00, 0.29, 10; 256:
+// 3.2, 2.2, 54.  8 qubits, 32: 2.2, 0.56, 6; 256: 16.5, 4.1, 6.  9 qubits, 32: 10,
+// 2.5, 2.  Gate by gate, 7 qubits, 8: 0.55, 0.31, 10; 256: 15.7, 9.3, 18; 8 qubits,
+// 256: 78, 17, 2.  Double-float, 8 qubits, 8: 0.47, 0.16, 11; 256: 6.8, 4.4, 52; 9
+// qubits, 256: 32, 14, 10.
 int default_wide(const dmsim_batch* b) {
-  if (b->mode == 0) return 7;
-  if (b->fused_arith) return 8;
-  int six = 0;
-  for (uint32_t n : b->nq) six += n == 6;
-  return six <= 8 ? 6 : 7;
+  auto at_most = [&](uint32_t n, int few) { return std::count(b->nq.begin(), b->nq.end(), n) <= few; };
+  if (b->mode == 0) return at_most(7, 8) ? 7 : 8;
+  if (b->fused_arith) return at_most(8, 8) ? 8 : 9;
+  if (!at_most(7, 32)) return 8;
+  return at_most(6, 8) ? 6 : 7;
 }
 
 void upload(dmsim_batch* b) {

@@ -230,8 +230,9 @@ typedef struct dmsim_batch* dmsim_batch_handle;
  * out (failure detection without a GPU fault). */
 enum { DMSIM_BATCH_OPT_WAIT_LIMIT = 100, DMSIM_BATCH_OPT_TEST_STALL = 101,
        /* circuits of at least this many qubits run on the engine's own pass kernels (tensor-core passes
-          included), as concurrent branches of the batch's graph; the rest share the work-queue kernel [unset: 6 or 7 by
-          the number of circuits, 7 for gate-by-gate batches, 8 for double-float ones] */
+          included), as concurrent branches of the batch's graph; the rest share the work-queue kernel [unset: 6, 7 or
+          8 by how many circuits there are of 6 and of 7 qubits; 7 or 8 for gate-by-gate batches, 8 or 9 for
+          double-float ones] */
        DMSIM_BATCH_OPT_WIDE_QUBITS = 102 };
 int dmsim_batch_create(uint32_t n_circuits, const uint32_t* n_qubits, dmsim_batch_handle* out);
 int dmsim_batch_destroy(dmsim_batch_handle b);

@@ -1,4 +1,5 @@
-"""What a batch's wide circuits cost outside its graph."""
+"""What a batch's wide circuits cost outside its graph, and how many narrow
+circuits stay with the work queue by default."""
 import time
 
 import numpy as np
@@ -30,3 +31,12 @@ def test_run_costs_no_copy_per_wide_circuit(engine):
             rest.append((time.perf_counter() - t) * 1e3 - b.stats()["ms"])
     assert np.median(rest) <= 0.5, rest
 
+
+@pytest.mark.parametrize("mode,arith,n,few", [("fused", "fp64", 6, 8), ("fused", "fp64", 7, 32), ("plain", "fp64", 7, 8),
+                                              ("fused", "df64", 8, 8)])
+def test_many_narrow_circuits_go_to_the_queue(engine, mode, arith, n, few):
+    for count in (few, few + 1):
+        with make(engine, [n] * count, mode=mode, fused_arith=arith) as b:
+            assert (b.stats()["items"] > 0) == (count > few)  # items: tiles of the queue
+            b.run()
+            assert abs(b.diag(count - 1).sum() - 1) <= 1e-9
