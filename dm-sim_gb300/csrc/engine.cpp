@@ -652,12 +652,18 @@ void run(dmsim_sim* s) {
   if (half) {
     // rho as the engine left it is Hermitian; after dmsim_set_dm or with the
     // device pointers handed out it is compared with its transpose first
-    // (one read of the state), unless the plan would save less than that
-    const double check_us = 6 + 2.0 * (double)s->N * (double)esize(s) / 5.0e6;
+    // (one read of the state), where the plan would save clearly more than that:
+    // half as much again, or four times as much for a state that fits L2, which
+    // saves less than half_gain_us says (CX passes on a Hermitian state that was
+    // written, with the check and whole: 11 qubits, 4 passes 93 and 77 us, 6 passes
+    // 119 and 108; 12 qubits, 4 passes 350 and 387; 13 qubits, 4 passes 1.15 and 1.40 ms)
+    const double state = 2.0 * (double)s->N * (double)esize(s);
+    const double check_us = 6 + state / 5.0e6;
+    const double margin = state <= 100e6 ? 4 : 1.5;
     if (s->herm_known && !s->exposed) {
       if (s->herm_flag != 1) DM_CUDA(launch_set_flag(s->d_herm, 1, s->stream));
       s->herm_flag = 1;
-    } else if (s->half_gain_us > check_us) {
+    } else if (s->half_gain_us > margin * check_us) {
       DM_CUDA(launch_check_hermitian(s->d_re, s->d_im, (int)s->n, s->d_herm, s->sms, s->stream));
       s->herm_flag = -1;
     } else {
