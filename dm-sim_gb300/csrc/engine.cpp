@@ -90,7 +90,9 @@ struct dmsim_sim {
   int arith = 0;        // arithmetic of the uploaded plan (kernels.h Arith)
   int64_t seed = -1;
 
-  double last_ms = 0, last_bytes = 0, predicted_ms = 0;
+  double last_ms = 0, predicted_ms = 0;
+  double last_bytes[2] = {0, 0};  // of the last run, whole and as planned
+  int ran_half = 0;               // 1: its half-range passes ran on half of rho; -1: as its check found, in *d_herm
   std::vector<PassRecord> records;
   std::string err;
 };
@@ -358,8 +360,8 @@ size_t plan_half_ranges(dmsim_sim* s, const std::vector<HalfCost>& costs,
     p.half = S[i];
     p.stale = stale;
     // bytes: the half range of the pass, and the mirror before it
-    if (p.half) p.bytes *= 0.5 * (1.0 + std::ldexp(1.0, -std::min(kHalfMaxS, __builtin_popcount(p.half))));
-    if (stale != p.half && stale) p.bytes += p.half ? part : full;
+    if (p.half) p.bytes[1] *= 0.5 * (1.0 + std::ldexp(1.0, -std::min(kHalfMaxS, __builtin_popcount(p.half))));
+    if (stale != p.half && stale) p.bytes[1] += p.half ? part : full;
     stale = p.half;
     if (!p.half) continue;
     const auto key = std::make_pair(p.half, geo[i]);
@@ -374,7 +376,7 @@ size_t plan_half_ranges(dmsim_sim* s, const std::vector<HalfCost>& costs,
     p.half_off = it->second;
   }
   s->end_stale = stale;
-  if (stale) s->passes.back().bytes += full;
+  if (stale) s->passes.back().bytes[1] += full;
   return total;
 }
 
@@ -404,7 +406,8 @@ void capture_passes(dmsim_sim* s) {
 // each a warp in FP64, fewer in double-float and FP32.  By itself a pass has four
 // times the threads, which small states need.
 struct MergeCost {
-  double apart = 0, pipe = 0, bytes = 0;  // the passes one by one; the sweep's pipe time; their bytes
+  double apart = 0, pipe = 0;  // the passes one by one; the sweep's pipe time
+  double bytes[2] = {0, 0};    // their bytes, whole and as planned
 };
 void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double frac, MergeCost& c) {
   double ops = 0;
@@ -418,10 +421,10 @@ void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double
   const double us = ops * 0.0333 * (fp64 ? 1 : 0.3);
   const double warps = frac * std::ldexp(1.0, 2 * (int)s->n - 2) / 32 / (4.0 * s->sms);  // of a 1-qubit pass, per scheduler
   // (a 2-qubit channel's tiles take twice their pipe's time by themselves)
-  c.apart += 1.8 + std::max(std::max(1.0, warps) * us / (op.kind == MO_CHANNEL2 ? 2 : 4), p.bytes / 5.8e6);
+  c.apart += 1.8 + std::max(std::max(1.0, warps) * us / (op.kind == MO_CHANNEL2 ? 2 : 4), p.bytes[1] / 5.8e6);
   // (FP64 dense operators and channels ran half as fast again in the sweep's few warps)
   c.pipe += std::max(1.0, warps / 4) * us * (fp64 && (op.kind == MO_DENSE || op.kind == MO_REAL || op.kind == MO_CHANNEL) ? 1.5 : 1);
-  c.bytes += p.bytes;
+  for (int w = 0; w < 2; w++) c.bytes[w] += p.bytes[w];
 }
 
 // Runs of consecutive passes that act on two qubits between them go in one sweep
@@ -442,11 +445,11 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
     size_t j = i;
     const uint32_t half = s->passes[i].half;
     const double frac = half ? 0.5 * (1.0 + std::ldexp(1.0, -std::min(kHalfMaxS, __builtin_popcount(half)))) : 1.0;
-    const double together = frac * 4.0 * (double)s->N * (double)esize(s);
+    const double whole = 4.0 * (double)s->N * (double)esize(s), together = frac * whole;  // bytes of a sweep
     MergeCost cost;
     // the best length so far: a run is cut where a longer one stops paying
     size_t best = 0;
-    double best_gain = 0, best_bytes = 0;
+    double best_gain = 0, best_bytes[2] = {0, 0};
     int best_q[2] = {-1, -1};
     for (; j < s->passes.size() && j - i < (size_t)kMultiOps; j++) {
       const PassInfo& p = s->passes[j];
@@ -465,7 +468,8 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
       if (j > i && gain > best_gain) {
         best = j - i + 1;
         best_gain = gain;
-        best_bytes = cost.bytes;
+        best_bytes[0] = cost.bytes[0];
+        best_bytes[1] = cost.bytes[1];
         best_q[0] = q[0];
         best_q[1] = q[1];
       }
@@ -490,7 +494,8 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
     total = off + sizeof(MultiDesc);
     PassInfo& p = s->passes[i];
     p.merged = (int)count;
-    p.multi_saved = std::max(0.0, best_bytes - together);
+    p.multi_saved[0] = std::max(0.0, best_bytes[0] - whole);
+    p.multi_saved[1] = std::max(0.0, best_bytes[1] - together);
     p.multi_off = off;
     if (half) {
       const size_t ho = (total + 15) & ~(size_t)15;
@@ -536,7 +541,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     std::memset(&pi, 0, sizeof pi);
     pi.conv = 1;
     pi.grid = (unsigned)s->sms * 8;
-    pi.bytes = conv_bytes;
+    pi.bytes[0] = conv_bytes;
     s->passes.push_back(pi);
     costs.push_back(whole);
     spec_of.push_back(-1);
@@ -549,7 +554,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       pi.transpose = true;
       pi.K = 0;
       pi.grid = (unsigned)s->sms * 8;
-      pi.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
+      pi.bytes[0] = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(pi);
       costs.push_back(whole);
       spec_of.push_back(-1);
@@ -571,7 +576,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     pi.cls = specs[i].cls;
     pi.desc_off = offs[i];
     pi.tile_entries = tile;
-    pi.bytes = (double)entries * 2.0 * (double)esize(s);
+    pi.bytes[0] = (double)entries * 2.0 * (double)esize(s);
     pi.nbasic = specs[i].nbasic;
     pi.feat.arith = arith;
     const int bps = pi.tc ? tc_blocks_per_sm(pi.K, arith) : pass_blocks_per_sm(pi.K, pi.cls, arith);
@@ -608,7 +613,7 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
       std::memset(&rn, 0, sizeof rn);
       rn.renorm = true;
       rn.grid = (unsigned)s->sms * 8;
-      rn.bytes = 2.0 * 2.0 * (double)s->N * (double)esize(s);
+      rn.bytes[0] = 2.0 * 2.0 * (double)s->N * (double)esize(s);
       s->passes.push_back(rn);
       costs.push_back(whole);
       spec_of.push_back(-1);
@@ -620,12 +625,13 @@ void upload_specs(dmsim_sim* s, const std::vector<PassSpec>& specs, uint32_t n_b
     std::memset(&pi, 0, sizeof pi);
     pi.conv = 2;
     pi.grid = (unsigned)s->sms * 8;
-    pi.bytes = conv_bytes;
+    pi.bytes[0] = conv_bytes;
     s->passes.push_back(pi);
     costs.push_back(whole);
     spec_of.push_back(-1);
     geo.push_back({});
   }
+  for (PassInfo& p : s->passes) p.bytes[1] = p.bytes[0];
   // complex64 runs stay whole: their renormalisation averages the two
   // partners' FP32 rounding errors, which a copied partner would not have
   // states below 10 qubits (16 MB) run whole too: their passes are launch and
@@ -647,8 +653,15 @@ void run(dmsim_sim* s) {
   if (!s->uploaded) throw DmError{DMSIM_ERR_STATE, "run() before upload()"};
   ensure_state(s);
   const bool timed = s->record != 0;
+  if (timed) {
+    for (PassInfo& p : s->passes) {
+      if (!p.ev0) DM_CUDA(cudaEventCreate(&p.ev0));
+      if (!p.ev1) DM_CUDA(cudaEventCreate(&p.ev1));
+    }
+  }
   bool half = false;
   for (const PassInfo& p : s->passes) half |= p.half != 0;
+  DM_CUDA(cudaEventRecord(s->ev0, s->stream));  // the run's time holds the check below
   if (half) {
     // rho as the engine left it is Hermitian; after dmsim_set_dm or with the
     // device pointers handed out it is compared with its transpose first
@@ -672,13 +685,6 @@ void run(dmsim_sim* s) {
     }
   }
   if (!s->keeps_herm) s->herm_known = false;
-  if (timed) {
-    for (PassInfo& p : s->passes) {
-      if (!p.ev0) DM_CUDA(cudaEventCreate(&p.ev0));
-      if (!p.ev1) DM_CUDA(cudaEventCreate(&p.ev1));
-    }
-  }
-  DM_CUDA(cudaEventRecord(s->ev0, s->stream));
   if (timed || !s->gexec) enqueue_passes(s, timed, s->stream, s->d_err);
   else DM_CUDA(cudaGraphLaunch(s->gexec, s->stream));
   DM_CUDA(cudaEventRecord(s->ev1, s->stream));
@@ -698,9 +704,13 @@ void run(dmsim_sim* s) {
   float ms = 0;
   DM_CUDA(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
   s->last_ms = ms;
-  double bytes = 0;
-  for (const PassInfo& p : s->passes) bytes += p.bytes - (timed ? 0 : p.multi_saved);
-  s->last_bytes = bytes;
+  s->ran_half = half ? s->herm_flag : 0;
+  for (int w = 0; w < 2; w++) {
+    s->last_bytes[w] = 0;
+    for (const PassInfo& p : s->passes) s->last_bytes[w] += p.bytes[w] - (timed ? 0 : p.multi_saved[w]);
+  }
+  // a check that passed read the whole state
+  if (s->ran_half < 0) s->last_bytes[1] += 2.0 * (double)s->N * (double)esize(s);
   if (timed) {
     s->records.clear();
     for (const PassInfo& p : s->passes) {
@@ -712,7 +722,7 @@ void run(dmsim_sim* s) {
       else if (p.transpose) r.feat.cls = kRecTranspose;
       else if (p.renorm) r.feat.cls = kRecRenorm;
       r.ms = pms;
-      r.bytes = p.bytes;
+      for (int w = 0; w < 2; w++) r.bytes[w] = p.bytes[w];
       r.grid = p.grid;
       s->records.push_back(r);
     }
@@ -725,6 +735,16 @@ void run(dmsim_sim* s) {
            s->n, s->circuit.size(), (double)ms, 0.0, (double)ms, mem, mem);
     printf("=====================================\n");
   }
+}
+
+// Whether the half-range passes of the last run ran on half of rho: 1 or 0.
+int ran_half(dmsim_sim* s) {
+  if (s->ran_half < 0) {
+    int flag = 0;
+    DM_CUDA(cudaMemcpy(&flag, s->d_herm, sizeof flag, cudaMemcpyDeviceToHost));
+    s->ran_half = flag != 0;
+  }
+  return s->ran_half;
 }
 
 void clear_circuit(dmsim_sim* s) {
@@ -1212,13 +1232,14 @@ int dmsim_last_timings(dmsim_handle s, double out[3]) {
     if (!out) throw DmError{DMSIM_ERR_ARG, "null output"};
     out[0] = s->last_ms;
     out[1] = (double)s->passes.size();
-    out[2] = s->last_bytes;
+    out[2] = s->last_bytes[ran_half(s)];
   });
 }
 
 int dmsim_pass_records(dmsim_handle s, double* out, uint32_t cap, uint32_t* count) {
   DM_TRY(s, {
     if (count) *count = (uint32_t)s->records.size();
+    const int half = ran_half(s);
     if (out)
       for (uint32_t i = 0; i < cap && i < s->records.size(); i++) {
         const PassRecord& r = s->records[i];
@@ -1230,7 +1251,7 @@ int dmsim_pass_records(dmsim_handle s, double* out, uint32_t cap, uint32_t* coun
         o[4] = r.feat.min_hi_bit;
         o[5] = r.feat.n;
         o[6] = r.ms;
-        o[7] = r.bytes;
+        o[7] = r.bytes[half];
         o[8] = r.feat.tc;
         o[9] = r.grid;
       }
@@ -1619,7 +1640,7 @@ cudaError_t sim_enqueue(dmsim_handle s, cudaStream_t st, int* err_word, std::str
 
 double sim_plan_bytes(dmsim_handle s) {
   double t = 0;
-  for (const PassInfo& p : s->passes) t += p.bytes - p.multi_saved;
+  for (const PassInfo& p : s->passes) t += p.bytes[1] - p.multi_saved[1];
   return t;
 }
 

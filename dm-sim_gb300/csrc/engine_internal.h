@@ -18,7 +18,8 @@ struct PassInfo {
   size_t desc_off;      // byte offset of the descriptor in the device blob
   int tile_entries;
   unsigned grid;
-  double bytes;         // algorithmic bytes moved (reads + writes)
+  double bytes[2];      // algorithmic bytes moved (reads + writes): run on the whole state, and as planned
+                        // (half range where `half`, with the mirror passes)
   int nbasic;
   bool tc;              // runs on the tensor cores (tensor.cu)
   bool hadamard;        // kPassHadamard pass (pass.h)
@@ -28,7 +29,7 @@ struct PassInfo {
   int merged;           // > 1: launched with the merged - 1 passes after it, in one sweep (kernels_multi.cu)
   size_t multi_off, multi_half_off;  // its MultiDesc and HalfMap in the device blob
   unsigned multi_grid;
-  double multi_saved;   // bytes that the sweep moves less than its passes one by one
+  double multi_saved[2];  // bytes that the sweep moves less than its passes one by one, whole and as planned
   int q0;               // first target qubit
   uint32_t half;        // half-range pass: its qubit set S (0: the whole state)
   uint32_t stale;       // the set under which the state is up to date before the pass: a mirror pass goes first
@@ -43,7 +44,7 @@ constexpr int kRecConvert = 16, kRecTranspose = 17, kRecRenorm = 18;
 struct PassRecord {
   PassFeatures feat;
   double ms;
-  double bytes;
+  double bytes[2];      // as PassInfo
   unsigned grid;
 };
 

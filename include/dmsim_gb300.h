@@ -132,7 +132,9 @@ int dmsim_n_gates(dmsim_handle h, uint32_t* n);
 int dmsim_plan_stats(dmsim_handle h, uint32_t* n_passes, uint32_t* n_basic);
 /* Bytes the last upload() copied to the device (the pass descriptors) */
 int dmsim_upload_bytes(dmsim_handle h, uint64_t* bytes);
-/* Timing of the last run: out[0] = ms, out[1] = passes, out[2] = bytes moved (algorithmic) */
+/* Timing of the last run: out[0] = ms, out[1] = passes, out[2] = bytes moved (algorithmic).  Both hold the check
+ * of a written rho (DMSIM_OPT_HERMITIAN) and count the range that the passes ran on: about half the bytes of a
+ * run in full show that rho was Hermitian. */
 int dmsim_last_timings(dmsim_handle h, double out[3]);
 /* Per-pass records of the last recorded run (DMSIM_OPT_RECORD): for each pass
  * DMSIM_PASS_RECORD doubles {K, class, nnz, max_lo_bit, min_hi_bit, n, ms,
