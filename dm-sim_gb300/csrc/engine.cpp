@@ -429,18 +429,21 @@ void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double
 
 // Runs of consecutive passes that act on two qubits between them go in one sweep
 // (kernels_multi.cu), their descriptors appended to the blob.  spec_of: the plan
-// entry of each pass, -1 for those that apply no gates.
+// entry of each pass, -1 for those that apply no gates; their descriptors stand at
+// p.desc_off of the blob.
 size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std::vector<int>& spec_of,
                     std::vector<unsigned char>& blob, size_t total) {
   const int n = (int)s->n;
   const bool had = s->arith == AR_FP64;
-  auto takes = [&](size_t i, int qa, int qb, MultiOp* op) {
-    const PassInfo& p = s->passes[i];
-    if (spec_of[i] < 0 || p.tc || (p.K == 1 && !p.direct1) || p.K > 2) return false;
-    return multi_op(specs[spec_of[i]], qa, qb, had, op);
-  };
+  // each pass's op, found once (a pass is tried in several runs)
+  std::vector<char> takes(s->passes.size());
+  std::vector<MultiOp> ops(s->passes.size());
   for (size_t i = 0; i < s->passes.size(); i++) {
-    MultiOp op;
+    const PassInfo& p = s->passes[i];
+    takes[i] = spec_of[i] >= 0 && !p.tc && p.K <= 2 && (p.K != 1 || p.direct1) &&
+               multi_op(specs[spec_of[i]], blob.data() + p.desc_off, had, &ops[i]);
+  }
+  for (size_t i = 0; i < s->passes.size(); i++) {
     int q[2] = {-1, -1};
     size_t j = i;
     const uint32_t half = s->passes[i].half;
@@ -454,7 +457,7 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
     for (; j < s->passes.size() && j - i < (size_t)kMultiOps; j++) {
       const PassInfo& p = s->passes[j];
       if (j > i && (p.half != s->passes[i].half || p.stale != p.half)) break;
-      if (!takes(j, -1, -1, &op)) break;
+      if (!takes[j]) break;
       const PassSpec& sp = specs[spec_of[j]];
       int u[4] = {q[0], q[1], -1, -1}, nu = (q[0] >= 0) + (q[1] >= 0);
       for (int k = 0; k < sp.K; k++)
@@ -462,7 +465,7 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
       if (nu > 2) break;
       q[0] = u[0];
       q[1] = u[1];
-      merge_cost(s, p, op, frac, cost);
+      merge_cost(s, p, ops[j], frac, cost);
       const double mem = together / 5.5e6;
       const double gain = 0.9 * cost.apart - (2.0 + std::max(cost.pipe, mem) + 0.3 * std::min(cost.pipe, mem));
       if (j > i && gain > best_gain) {
@@ -490,7 +493,10 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
     d->nops = (int)count;
     d->qa = qa;
     d->qb = qb;
-    for (size_t k = 0; k < count; k++) takes(i + k, qa, qb, &d->op[k]);
+    for (size_t k = 0; k < count; k++) {
+      d->op[k] = ops[i + k];
+      d->op[k].p = specs[spec_of[i + k]].q[ops[i + k].p] == qa ? 0 : 1;
+    }
     total = off + sizeof(MultiDesc);
     PassInfo& p = s->passes[i];
     p.merged = (int)count;

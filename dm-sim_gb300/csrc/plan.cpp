@@ -2,6 +2,7 @@
 #include "plan.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -781,7 +782,7 @@ uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uin
 }
 
 // ---------------------------------------------------------------- several passes in one sweep
-bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
+bool multi_op(const PassSpec& p, const void* desc, bool hadamard, MultiOp* out) {
   if (p.transpose || p.rlin || p.ket_only || p.K < 1 || p.K > 2) return false;
   std::memset(out, 0, sizeof *out);
   if (p.K == 2 && p.super) {
@@ -795,7 +796,6 @@ bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
         if (term) out->c[od ? (o / 4) * 4 + j / 4 : 16 + o] = m.real();
       }
     out->kind = MO_CHANNEL2;
-    out->p = p.q[0] == qa ? 0 : 1;
     return true;
   }
   if (p.K == 2) {
@@ -809,12 +809,11 @@ bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
       }
       if (!cx) continue;
       out->kind = MO_CX;
-      out->p = p.q[c] == qa ? 0 : 1;
+      out->p = c;
       return true;
     }
     return false;
   }
-  out->p = p.q[0] == qa ? 0 : 1;
   if (p.super) {
     // the register kernel's simple channels
     uint32_t nz = 0;
@@ -830,17 +829,16 @@ bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out) {
     out->flags = (int)diag | (cross ? 4 : 0);
     return true;
   }
-  std::unique_ptr<PassDesc<1>> d(new PassDesc<1>);
-  build_k<1>(p, 17, d.get(), nullptr, nullptr, nullptr, 8);  // factors, kinds and flags: the same for every size
-  const PassOp<1>& op = d->op;
+  const PassDesc<1>& d = *static_cast<const PassDesc<1>*>(desc);
+  const PassOp<1>& op = d.op;
   if (p.cls == CLS_DENSE || p.cls == CLS_SPARSE) {
     if (p.cls == CLS_SPARSE) return false;
-    if (hadamard && (d->h.flags & kPassHadamard)) {
+    if (hadamard && (d.h.flags & kPassHadamard)) {
       out->kind = MO_HADAMARD;
       out->flags = (op.ure[0] * op.ure[1] < 0 ? 1 : 0) | (op.ure[0] * op.ure[2] < 0 ? 2 : 0);
       return true;
     }
-    out->kind = d->h.flags & kPassRealOperator ? MO_REAL : MO_DENSE;
+    out->kind = d.h.flags & kPassRealOperator ? MO_REAL : MO_DENSE;
     for (int i = 0; i < 4; i++) {
       out->c[i] = op.ure[i];
       out->c[4 + i] = op.uim[i];
@@ -917,11 +915,7 @@ double pass_us(const HalfCost& c, int s) {
   const double f = s == 0 ? 1.0 : 0.5 * (1.0 + std::ldexp(1.0, -s));
   return c.fixed_us + c.tile_us * std::max(1.0, std::ceil(c.tiles * f / c.slots));
 }
-int count_bits(uint32_t m) {
-  int c = 0;
-  for (; m; m &= m - 1) c++;
-  return std::min(c, kHalfMaxS);
-}
+int count_bits(uint32_t m) { return std::min(__builtin_popcount(m), kHalfMaxS); }
 }  // namespace
 
 std::vector<uint32_t> plan_half(const std::vector<HalfCost>& passes, double part_us, double full_us, double* gain_us) {
@@ -935,9 +929,12 @@ std::vector<uint32_t> plan_half(const std::vector<HalfCost>& passes, double part
   std::vector<int> from(m + 1, -1);
   std::vector<char> from_half(m + 1, 0), full_from_half(m + 1, 0);
   f[0] = 0;
+  std::vector<std::array<double, kHalfMaxS + 1>> us(m);  // of each pass, per |S|
+  for (int i = 0; i < m; i++)
+    for (int s = 0; s <= kHalfMaxS; s++) us[i][s] = pass_us(passes[i], s);
   double all = 0;
   for (int i = 0; i < m; i++) {
-    const double t = pass_us(passes[i], 0);
+    const double t = us[i][0];
     all += t;
     const double a = f[i] + t, b = h[i] + full_us + t;
     if (std::min(a, b) < f[i + 1]) {
@@ -946,14 +943,19 @@ std::vector<uint32_t> plan_half(const std::vector<HalfCost>& passes, double part
     }
     const double start = std::min(f[i], h[i] + part_us);
     const bool start_half = h[i] + part_us < f[i];
-    uint32_t S = ~0u;
+    uint32_t S = ~0u, counted = 0;
+    int bits = 0;  // of S, at most kHalfMaxS
     // per |S| the time of the stretch so far
     double sum[kHalfMaxS + 1] = {0};
     for (int j = i; j < m && j < i + kReach; j++) {
       S &= passes[j].allowed;
       if (S == 0) break;
-      for (int s = 1; s <= kHalfMaxS; s++) sum[s] += pass_us(passes[j], s);
-      const double c = start + sum[count_bits(S)];
+      if (S != counted) {
+        counted = S;
+        bits = count_bits(S);
+      }
+      for (int s = 0; s <= kHalfMaxS; s++) sum[s] += us[j][s];
+      const double c = start + sum[bits];
       if (c < h[j + 1]) {
         h[j + 1] = c;
         from[j + 1] = i;

@@ -83,8 +83,9 @@ size_t tc_desc_bytes(int K, int arith = 2);
 uint64_t build_tc_desc(const PassSpec& p, int n, void* out, PassFeatures* f, uint64_t* ntiles, int* tile_entries,
                        bool slices = true, int arith = 2);
 // ---- several narrow passes in one sweep (pass.h): whether a pass can take part,
-// and its op, with its qubits as 0 (qa) and 1 (qb).
-bool multi_op(const PassSpec& p, int qa, int qb, bool hadamard, MultiOp* out);
+// and its op, out->p the index into p.q of the qubit that it names.  d: its
+// descriptor (K = 1: PassDesc<1>).
+bool multi_op(const PassSpec& p, const void* d, bool hadamard, MultiOp* out);
 // ---- half-range passes (pass.h)
 // The qubits that a pass's tiles have one ket and one bra value of: the set S
 // of a half-range pass is drawn from them.  Tiled passes: not targets, and
