@@ -25,8 +25,11 @@
 // 6 and 7 floored at 2^-43 of order 0) and the bra step's result is rounded
 // once to FP64 from the 64-bit integer.  Each value is held with 55 significant
 // bits relative to its column's largest (block floating point per column of
-// 2^K entries): the error of an output is below 2^-54 of its operator row's
-// 1-norm times its column's largest value, per step.
+// 2^K entries), an operator's entry relative to its row's largest.  The error of
+// an output, per step, X its column's largest value, w its row: at most one unit
+// (2^-54 X) a value (the conversions err by half of one, the shifts by one), half
+// a unit (2^-55 max|w|) an entry, and the orders that are left out and floored:
+// 2^-54 X (|w|_1 + (1.04 D + 1) max|w|), D = 2^K.
 //
 // Threads: 1024 (32 warps, 64 registers each), one block per SM, as two
 // independent groups of 16 warps that take alternate tiles of the block, each
