@@ -23,8 +23,6 @@ namespace {
 __device__ __forceinline__ double xor_sign(double x, bool n) {
   return __hiloint2double(__double2hiint(x) ^ (n ? (int)0x80000000 : 0), __double2loint(x));
 }
-__device__ __forceinline__ float xor_sign(float x, bool n) { return n ? -x : x; }
-__device__ __forceinline__ df64 xor_sign(df64 x, bool n) { return n ? -x : x; }
 
 template <typename T, int CLS_, bool HALF>
 __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict__ im,
@@ -326,7 +324,8 @@ cudaError_t launch1_t(const LaunchArgs& a, cudaStream_t s) {
     case CLS_SIGNED: return launch1<T, CLS_SIGNED>(a, s);
     case CLS_PHASE: return launch1<T, CLS_PHASE>(a, s);
     case CLS_DENSE:
-      if (a.hadamard && std::is_same<T, double>::value) return launch1<T, CLS_HADAMARD>(a, s);
+      if constexpr (std::is_same<T, double>::value)
+        if (a.hadamard) return launch1<T, CLS_HADAMARD>(a, s);
       return a.real ? launch1<T, CLS_DENSE_REAL>(a, s) : launch1<T, CLS_DENSE>(a, s);
     case CLS_SUPER: return launch1<T, CLS_SUPER>(a, s);
     default: return cudaErrorInvalidValue;

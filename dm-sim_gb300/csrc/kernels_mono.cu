@@ -218,12 +218,11 @@ cudaError_t launch_mono_t(const LaunchArgs& a, cudaStream_t s) {
 
 // A tile for every block: at 10 qubits (1024 tiles) a CX takes 12.0 us, 12.4 on
 // the tiled kernel; below, blocks would find their positions for no tile.
-constexpr uint64_t kMonoTiles = 1;
 unsigned mono_grid(int K, int cls, int tile_entries, uint64_t ntiles, int sms) {
   if (K < 2 || K > 4 || tile_entries != 256 << K) return 0;
   if (cls != CLS_MOVE && cls != CLS_SIGNED && cls != CLS_PHASE) return 0;
   const uint64_t cap = (uint64_t)sms * (K <= 3 ? 2 : 1);
-  return ntiles >= kMonoTiles * cap ? (unsigned)cap : 0;
+  return ntiles >= cap ? (unsigned)cap : 0;
 }
 
 cudaError_t launch_mono(const LaunchArgs& a, cudaStream_t s) {

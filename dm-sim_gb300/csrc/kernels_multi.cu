@@ -126,24 +126,26 @@ __device__ __forceinline__ void apply1(const OpShared<T>& op, T (&xr)[16], T (&x
       dense4<T, true>(op, r0, r1, r2, r3, i0, i1, i2, i3);
     });
   } else if (kind == MO_HADAMARD) {
-    each_group<T, P>(xr, xi, [&](T& r0, T& r1, T& r2, T& r3, T& i0, T& i1, T& i2, T& i3) {
-      auto h = [](T& x0, T& x1, T& x2, T& x3) {
-        const T s0 = x0 + x1, d0 = x0 - x1, s1 = x2 + x3, d1 = x2 - x3;
-        x0 = half_of(s0 + s1);
-        x1 = half_of(d0 + d1);
-        x2 = half_of(s0 - s1);
-        x3 = half_of(d0 - d1);
-      };
-      h(r0, r1, r2, r3);
-      h(i0, i1, i2, i3);
-      if (fl & 2) r1 = flip(r1), r2 = flip(r2), i1 = flip(i1), i2 = flip(i2);
-      if (fl & 1) {
-        swap2(r0, r3);
-        swap2(r1, r2);
-        swap2(i0, i3);
-        swap2(i1, i2);
-      }
-    });
+    if constexpr (std::is_same<T, double>::value) {  // FP64 only, as its passes by themselves
+      each_group<T, P>(xr, xi, [&](T& r0, T& r1, T& r2, T& r3, T& i0, T& i1, T& i2, T& i3) {
+        auto h = [](T& x0, T& x1, T& x2, T& x3) {
+          const T s0 = x0 + x1, d0 = x0 - x1, s1 = x2 + x3, d1 = x2 - x3;
+          x0 = half_of(s0 + s1);
+          x1 = half_of(d0 + d1);
+          x2 = half_of(s0 - s1);
+          x3 = half_of(d0 - d1);
+        };
+        h(r0, r1, r2, r3);
+        h(i0, i1, i2, i3);
+        if (fl & 2) r1 = flip(r1), r2 = flip(r2), i1 = flip(i1), i2 = flip(i2);
+        if (fl & 1) {
+          swap2(r0, r3);
+          swap2(r1, r2);
+          swap2(i0, i3);
+          swap2(i1, i2);
+        }
+      });
+    }
   } else if (kind == MO_MONO) {
     each_group<T, P>(xr, xi, [&](T& r0, T& r1, T& r2, T& r3, T& i0, T& i1, T& i2, T& i3) {
       if (fl & 1) {

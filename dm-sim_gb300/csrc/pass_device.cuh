@@ -170,8 +170,6 @@ __device__ __forceinline__ double half_of(double x) {
   if (e == 0x00100000u || e == 0x7FF00000u || (e == 0 && ((h << 1) | l))) return 0.5 * x;
   return __hiloint2double(h - (e ? 0x00100000 : 0), l);
 }
-__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
-__device__ __forceinline__ df64 half_of(df64 x) { return df64(0.5f * x.hi, 0.5f * x.lo); }
 
 template <int K>
 __device__ __forceinline__ int pext_local(int loc, const int* lpos) {
