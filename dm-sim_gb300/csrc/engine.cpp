@@ -993,8 +993,9 @@ int dmsim_append_c2(dmsim_handle s, uint32_t q1, uint32_t q2, const double m[32]
 
 namespace {
 // Kraus operators -> the superoperator S = sum_i K_i (x) conj(K_i) in the pass
-// sub-index order (bit i <-> qubit q[i]); the caller's 2-qubit matrices use the
-// C2 basis order (index 2*bit(q1) + bit(q2)), so the two bits are swapped here.
+// sub-index order (bit i <-> the pass's qubit i).  The caller's 2-qubit matrices
+// are on the index bit(q[0]) + 2 bit(q[1]); the pass's first qubit is q[1], so the
+// two bits are swapped.
 void append_kraus(dmsim_sim* s, uint32_t nq, const uint32_t q[2], uint32_t nk, const cplx* kraus) {
   if (nq < 1 || nq > 2) throw DmError{DMSIM_ERR_ARG, "channels act on 1 or 2 qubits"};
   if (nk < 1 || nk > 16) throw DmError{DMSIM_ERR_ARG, "1 to 16 Kraus operators"};
@@ -1004,7 +1005,7 @@ void append_kraus(dmsim_sim* s, uint32_t nq, const uint32_t q[2], uint32_t nk, c
   g.nq = (int)nq;
   if (nq == 1) g.qb[0] = q[0];
   else {
-    g.qb[0] = q[1];  // pass sub-index bit 0 <-> the caller's second qubit
+    g.qb[0] = q[1];  // the pass's first qubit
     g.qb[1] = q[0];
   }
   check_qubits(s, g);

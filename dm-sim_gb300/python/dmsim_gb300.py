@@ -207,8 +207,9 @@ class Simulation:
         self._check(lib().dmsim_append_c2(self._h, int(q1), int(q2), _dp(flat)))
 
     def append_channel(self, qubits, kraus):
-        """rho -> sum_i K_i rho K_i^+ on 1 or 2 qubits (2-qubit matrices in the
-        C2 basis order, index 2*bit(qubits[0]) + bit(qubits[1]))."""
+        """rho -> sum_i K_i rho K_i^+ on 1 or 2 qubits.  2-qubit matrices are on
+        the index bit(qubits[0]) + 2*bit(qubits[1]): np.kron(A, B) is A on
+        qubits[1] and B on qubits[0] (append_c2's index is the other way round)."""
         qs = list(qubits)
         k = np.asarray(kraus, dtype=np.complex128).reshape(len(kraus), -1)
         flat = np.empty(2 * k.size)

@@ -90,8 +90,10 @@ int dmsim_append_c2(dmsim_handle h, uint32_t q1, uint32_t q2, const double m[32]
 /* Noise channel (no counterpart in the reference, which has no noise):
  * rho -> sum_i K_i rho K_i^+ on nq = 1 or 2 qubits q[0..nq-1]; kraus holds
  * n_kraus (<= 16) matrices of 2^nq x 2^nq complex, row-major, re/im
- * interleaved, 2-qubit ones in the C2 basis order (index 2*bit(q[0]) +
- * bit(q[1])).  Applied as one superoperator pass; a fusion barrier. */
+ * interleaved, 2-qubit ones on the index bit(q[0]) + 2*bit(q[1]): A (x) B
+ * (row 2i + j of A's row i, B's row j) is A on q[1] and B on q[0], the reverse
+ * of dmsim_append_c2's order.  Applied as one superoperator pass; a fusion
+ * barrier. */
 int dmsim_append_channel(dmsim_handle h, uint32_t nq, const uint32_t q[2], uint32_t n_kraus, const double* kraus);
 enum dmsim_noise {
   DMSIM_NOISE_DEPOLARIZING = 0,       /* rho -> (1-p) rho + p I/2 */
