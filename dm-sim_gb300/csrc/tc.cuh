@@ -1,11 +1,12 @@
 // tc.cuh -- the Blackwell tensor-core primitives the tensor passes use, as
 // inline PTX for sm_100a/sm_103a: tensor-memory (TMEM) allocation, tcgen05.mma
-// (kind::f16, BF16 operands from shared memory, FP32 accumulators in TMEM),
+// (kind::f16, both operands BF16 or both FP16, from shared memory, FP32
+// accumulators in TMEM),
 // tcgen05.commit to an mbarrier, tcgen05.ld of the accumulators, and the
 // fences that order them against ordinary shared-memory traffic.
 //
-// Operand layout: K-major, no swizzle.  A row-major M x K (or N x K) BF16
-// matrix is stored as 8-row x 16-byte "core matrices" (8 rows of 8 BF16, 128
+// Operand layout: K-major, no swizzle.  A row-major M x K (or N x K) 16-bit
+// matrix is stored as 8-row x 16-byte "core matrices" (8 rows of 8 values, 128
 // contiguous bytes); core matrices adjacent along K are kLbo bytes apart,
 // 8-row groups adjacent along M/N are `sbo` bytes apart.
 #pragma once

@@ -29,8 +29,9 @@
 // error flag, and the block releases its tensor memory; the host reports
 // DMSIM_ERR_TIMEOUT with rho undefined.
 //
-// What bounds it: issue (60 % active), the ALU and the load/store pipe (40 %
-// each), and the twelve small MMAs of a step, 140 cycles each.  A 4-qubit pass at
+// What bounds it: no pipe is full (12 qubits, ncu: issue 46 %, ALU 34 %, load/store
+// 31 %, tensor 12 %); a group's steps follow one another, with twelve small MMAs a
+// step, 140 cycles each.  A 4-qubit pass at
 // 15 qubits (8.6 GB read and as much written) takes 4.9 ms, 3.5 TB/s; 6.6 ms before the tiles
 // came in by 16-byte copies.  An accumulator for each order of the slice pairs (six
 // wider MMAs) took 4.7 ms and erred a sixth less, but other roundings than before

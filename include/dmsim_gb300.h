@@ -38,13 +38,15 @@ enum dmsim_option {
   DMSIM_OPT_PRECISION = 2,  /* 0 = FP64 [0], 1 = complex64 (FP32 passes, FP64 reductions); set before the first append */
   DMSIM_OPT_MAX_K = 3,      /* widest fused operator, 1..4 [4] */
   DMSIM_OPT_PLANNER = 4,    /* 0 = greedy fixed width [0], 1 = learned cost model */
-  DMSIM_OPT_RECORD = 5,     /* 1 = time every pass of the next runs (no graph) [0] */
+  DMSIM_OPT_RECORD = 5,     /* 1 = time every pass of the next runs, launched one by one: no graph, no merged
+                               sweeps, no overlapped launches, so the run takes longer than an unrecorded one [0] */
   DMSIM_OPT_SEED = 6,       /* seed of measure() without uniforms; -1 = time(0) like the reference [-1] */
   DMSIM_OPT_GRAPH = 7,      /* 1 = replay uploaded circuits from a captured CUDA graph [1] */
   DMSIM_OPT_VERBOSE = 8,    /* 1 = print the reference's per-run timing banner [0] */
   DMSIM_OPT_FUSED_ARITH = 9, /* fused FP64 runs: 0 = FP64 width [0] (3/4-qubit passes on the tensor cores with
                                  7 FP16 digits per operand and exact integer sums, the rest in FP64), 1 = double-float
-                                 passes on the FP32 pipe and tensor cores (48-bit significands) */
+                                 passes on the FP32 pipe and tensor cores (48-bit significands; less exact, and
+                                 slower than FP64 width at 14 qubits fused: 1.83 s against 1.59) */
   DMSIM_OPT_RENORM = 10,     /* complex64: FP64 trace + Hermitian renormalisation every R passes and at the end [64]; 0 = off */
   DMSIM_OPT_PLAIN_ARITH = 11, /* plain FP64 runs (FP64 state at rest): 0 = FP64 passes [0] (dense passes bound by
                                  GB300's FP64 pipe), 1 = double-float passes on the FP32 pipe (HBM-bound) */
@@ -53,11 +55,14 @@ enum dmsim_option {
                                  FP64-width run, the 4-qubit passes of a complex64 run (BF16 x 3 split, FP32
                                  accumulation) and, in double-float runs, passes above a density rule [1];
                                  0 = never; 2 = every eligible pass */
-  DMSIM_OPT_DIRECT1 = 13,     /* 1 = 1-qubit move/sign/phase/dense passes on the register kernel (no shared-memory
-                                 tiles) [1], 0 = the tiled kernel */
+  DMSIM_OPT_DIRECT1 = 13,     /* 1 = 1-qubit move/sign/phase/dense passes and channels on the register kernel (no
+                                 shared-memory tiles), and runs of narrow passes merged into one sweep [1], 0 = the
+                                 tiled kernel, nothing merged */
   DMSIM_OPT_HERMITIAN = 14    /* 1 = passes may compute one of every two Hermitian partners rho[r][c], rho[c][r] and
                                  copy the other [1]; a rho written through dmsim_set_dm or the device pointers is
-                                 first checked, and runs in full when it is not Hermitian; 0 = every pass in full */
+                                 first checked, entry by entry for equality, and runs in full when it is not
+                                 Hermitian or the plan is too short to gain from it (dmsim_last_timings' bytes
+                                 tell which); 0 = every pass in full */
 };
 
 /* Gate ids: the order of enum OP, src/dmsim_nvgpu_omp.cuh:42-48 (ABI). */
