@@ -29,7 +29,8 @@ namespace dmg {
 // FP32 pipe a dense row is 4 * 2^K multiply-adds fed by 16-byte broadcast
 // coefficient loads, where the sparse row walk costs several dependent
 // shared-memory loads per nonzero and runs slower at every density these
-// fused blocks have.  (FP64 and double-float keep the sparse walk: their
+// fused blocks have; the runs that such a pass does not load count as zeros
+// (kZeroUnloaded).  (FP64 and double-float keep the sparse walk: their
 // multiply-adds, not the loads, bound them.)
 template <typename T, int K>
 constexpr bool sparse_as_dense() {

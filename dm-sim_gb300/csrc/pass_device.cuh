@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "pass.h"
 
 namespace dmg {
@@ -366,6 +368,13 @@ __device__ __forceinline__ uint64_t tile_base(const PassHeader& h, const HalfMap
   return hm ? half_base(*hm, t, h.L) : tile_base(h, t);
 }
 
+// Whether the tile's runs that are not loaded have to be zeros in shared memory: a
+// complex64 DENSE instance of 3 or 4 qubits also runs SPARSE passes (kernels.cu),
+// whose load mask leaves out runs that only structural zeros would read -- and
+// 0 times whatever an earlier kernel left there may be NaN.
+template <typename T, int K, int CLS>
+constexpr bool kZeroUnloaded = std::is_same<T, float>::value && K >= 3 && CLS == CLS_DENSE;
+
 // Register staging of one tile's loads: thread tid holds entry pairs
 // tid + 256 i (i < P) -- the next tile's loads are issued before the current
 // tile is transformed, so their latency hides behind its arithmetic.
@@ -401,6 +410,9 @@ __device__ __forceinline__ void regs_to_smem(const PassHeader& h, const PassTabl
     if ((tb.ldmask[run >> 5] >> (run & 31)) & 1) {
       st_pair<T>(sre, e, x.r[k]);
       st_pair<T>(sim, e, x.i[k]);
+    } else if constexpr (kZeroUnloaded<T, K, CLS>) {
+      st_pair<T>(sre, e, T2{0, 0});
+      st_pair<T>(sim, e, T2{0, 0});
     }
   }
 }
@@ -425,7 +437,13 @@ __device__ void run_tile(T* __restrict__ re, T* __restrict__ im, const PassHeade
   for (int e2 = tid; e2 < (tile >> 1); e2 += blockDim.x) {
     const int e = e2 << 1;
     const int run = e >> L;
-    if (!((tb.ldmask[run >> 5] >> (run & 31)) & 1)) continue;
+    if (!((tb.ldmask[run >> 5] >> (run & 31)) & 1)) {
+      if constexpr (kZeroUnloaded<T, K, CLS>) {
+        st_pair<T>(sre, e, T2{0, 0});
+        st_pair<T>(sim, e, T2{0, 0});
+      }
+      continue;
+    }
     const uint64_t ga = base + tb.hioff[run] + (uint64_t)(e & (runlen - 1));
     const T2 vr = ld2<T>(re + ga);
     const T2 vi = ld2<T>(im + ga);
