@@ -164,10 +164,17 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
   // qubits fused 20.3 -> 19.9 ms; at 14 qubits the waiting blocks cost 3 %), and
   // only grids of at most one block an SM, of whole numbers of them (persistent
   // blocks) or of several: otherwise blocks placed around the running kernel's make
-  // uneven loads (9 qubits, 256 blocks: 565 -> 720).
+  // uneven loads (9 qubits, 256 blocks: 565 -> 720).  So do those of the tiled kernel
+  // on operators of 2 qubits and more (wide), whose tiles take long: it starts early
+  // with at most one block an SM, and FP64 ones of 3 and 4 qubits only where the
+  // kernel before leaves an SM to each (9 qubits, such passes off the tensor cores,
+  // 727 us without, 1183 with any overlap; complex64, 11 qubits, 3-qubit passes 1072
+  // and 1174; 12 qubits, 2-qubit passes 11 % less without).
   const bool overlap = !timed && s->n <= 12;
-  auto may_overlap = [&](unsigned grid) {
+  unsigned before = 0;  // blocks of the kernel that goes before
+  auto may_overlap = [&](unsigned grid, const PassInfo* wide) {
     const unsigned sms = (unsigned)s->sms;
+    if (wide) return grid <= sms && !(s->arith == AR_FP64 && wide->K >= 3 && before + grid > sms);
     return grid <= sms || grid % sms == 0 || grid >= 4 * sms;
   };
   bool pdl = false;  // a kernel of the sequence goes before
@@ -225,13 +232,14 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
       a.desc = static_cast<const char*>(s->d_desc) + p.multi_off;
       a.grid = p.multi_grid;
       a.half = p.half ? reinterpret_cast<const HalfMap*>(static_cast<const char*>(s->d_desc) + p.multi_half_off) : nullptr;
-      a.pdl = pdl && may_overlap(a.grid);
+      a.pdl = pdl && may_overlap(a.grid, nullptr);
       DM_CUDA(launch_multi(a, st));
       i += p.merged - 1;
     } else {
-      a.pdl = pdl && may_overlap(p.grid);
+      a.pdl = pdl && may_overlap(p.grid, !p.tc && !p.direct1 && !p.mono && p.K >= 2 ? &p : nullptr);
       DM_CUDA(launch_pass(a, st));
     }
+    before = a.grid;
     pdl = overlap;
     if (i + 1 == s->passes.size()) mirror(s->end_stale, 0, true);
     if (timed) DM_CUDA(cudaEventRecord(p.ev1, st));
