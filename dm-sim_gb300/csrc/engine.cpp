@@ -329,6 +329,14 @@ HalfCost half_cost(const dmsim_sim* s, const PassInfo& p, const PassSpec& spec, 
   c.slots = 1;
   c.tiles = 1000;  // no rounding: many small tiles
   c.tile_us = N * std::max(bw, fma * rate) * 1e-6 / c.tiles;
+  if (s->arith == AR_DF64 && p.K >= 3 && !p.mono) {
+    // wide double-float tiles: a block's steps wait for one another, so a round takes
+    // as long with half of the SMs' places filled (10 qubits, QFT and layers off the
+    // tensor cores, 908 us whole, 936 with half ranges chosen by the tiles' share)
+    c.slots = (double)s->sms * pass_blocks_per_sm(p.K, p.cls, s->arith);
+    c.tile_us *= c.tiles * c.slots / (double)ntiles;
+    c.tiles = (double)ntiles;
+  }
   return c;
 }
 
