@@ -439,7 +439,10 @@ void merge_cost(const dmsim_sim* s, const PassInfo& p, const MultiOp& op, double
   // (a 2-qubit channel's tiles take twice their pipe's time by themselves)
   c.apart += 1.8 + std::max(std::max(1.0, warps) * us / (op.kind == MO_CHANNEL2 ? 2 : 4), p.bytes[1] / 5.8e6);
   // (FP64 dense operators and channels ran half as fast again in the sweep's few warps)
-  c.pipe += std::max(1.0, warps / 4) * us * (fp64 && (op.kind == MO_DENSE || op.kind == MO_REAL || op.kind == MO_CHANNEL) ? 1.5 : 1);
+  // (a lone warp takes 2 us for a double-float 1-qubit channel: 8 qubits and less, 1.4
+  // to 1.8 us by itself, 2.0 to 2.1 in a sweep)
+  const double alone = s->arith == AR_DF64 && op.kind == MO_CHANNEL ? 2.0 : 0;
+  c.pipe += std::max(alone, std::max(1.0, warps / 4) * us * (fp64 && (op.kind == MO_DENSE || op.kind == MO_REAL || op.kind == MO_CHANNEL) ? 1.5 : 1));
   for (int w = 0; w < 2; w++) c.bytes[w] += p.bytes[w];
 }
 
@@ -458,6 +461,8 @@ size_t merge_passes(dmsim_sim* s, const std::vector<PassSpec>& specs, const std:
     const PassInfo& p = s->passes[i];
     takes[i] = spec_of[i] >= 0 && !p.tc && p.K <= 2 && (p.K != 1 || p.direct1) &&
                multi_op(specs[spec_of[i]], blob.data() + p.desc_off, had, &ops[i]);
+    // double-float dense operators on a lone warp: 5.8 us in a sweep, less by themselves
+    if (s->arith == AR_DF64 && n <= 4 && ops[i].kind == MO_DENSE) takes[i] = false;
   }
   for (size_t i = 0; i < s->passes.size(); i++) {
     int q[2] = {-1, -1};

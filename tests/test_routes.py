@@ -67,6 +67,18 @@ def test_narrow_passes_are_merged(engine, n, precision, arith, noise):
     assert merged < 0.7 * single
 
 
+@pytest.mark.parametrize("n,merged", [(3, False), (8, False), (10, True)])
+def test_double_float_channels_are_merged_where_it_pays(engine, n, merged):
+    """A lone warp takes longer for them in a sweep than a pass by itself."""
+    with engine.Simulation(n, mode="plain", plain_arith="df64") as s:
+        for i in range(12):
+            s.append_noise("depolarizing", (i & 1,), 0.1)
+        s.upload()
+        one = run_bytes(s)
+        s.set_option(engine.OPT_RECORD, 1)
+        assert (one < run_bytes(s)) == merged
+
+
 @pytest.mark.parametrize("kind,gate", [("move", "CX"), ("signed", "CZ"), ("phase", "CU1")])
 @pytest.mark.parametrize("n,precision,arith", [(10, "fp64", "fp64"), (11, "fp64", "df64"), (11, "c64", "fp64"), (12, "fp64", "fp64")])
 @pytest.mark.parametrize("k", [2, 3, 4])
