@@ -165,7 +165,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
   // only grids of at most one block an SM, of whole numbers of them (persistent
   // blocks) or of several: otherwise blocks placed around the running kernel's make
   // uneven loads (9 qubits, 256 blocks: 565 -> 720).  So do those of the tiled kernel
-  // on operators of 2 qubits and more (wide), whose tiles take long: it starts early
+  // on dense or sparse rows of 2 qubits and more (wide), whose tiles take long: it starts early
   // with at most one block an SM, and FP64 ones of 3 and 4 qubits only where the
   // kernel before leaves an SM to each (9 qubits, such passes off the tensor cores,
   // 727 us without, 1183 with any overlap; complex64, 11 qubits, 3-qubit passes 1072
@@ -176,6 +176,9 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
     const unsigned sms = (unsigned)s->sms;
     if (wide) return grid <= sms && !(s->arith == AR_FP64 && wide->K >= 3 && before + grid > sms);
     return grid <= sms || grid % sms == 0 || grid >= 4 * sms;
+  };
+  auto tiled_rows = [&](const PassInfo& p) {  // (complex64 circuits of 10 qubits lose 1 % by it)
+    return !p.tc && !p.direct1 && p.K >= 2 && (p.cls == CLS_DENSE || p.cls == CLS_SPARSE) && (!s->fp32 || s->n >= 11);
   };
   bool pdl = false;  // a kernel of the sequence goes before
   auto mirror = [&](uint32_t from, uint32_t to, bool last) {
@@ -236,7 +239,7 @@ void enqueue_passes(dmsim_sim* s, bool timed, cudaStream_t st, int* err_word) {
       DM_CUDA(launch_multi(a, st));
       i += p.merged - 1;
     } else {
-      a.pdl = pdl && may_overlap(p.grid, !p.tc && !p.direct1 && !p.mono && p.K >= 2 ? &p : nullptr);
+      a.pdl = pdl && may_overlap(p.grid, tiled_rows(p) ? &p : nullptr);
       DM_CUDA(launch_pass(a, st));
     }
     before = a.grid;

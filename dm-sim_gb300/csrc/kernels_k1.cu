@@ -34,9 +34,9 @@ __global__ void __launch_bounds__(256) k_pass1(T* __restrict__ re, T* __restrict
   constexpr bool kSuper = CLS == CLS_SUPER;
   constexpr bool kHad = CLS_ == CLS_HADAMARD;
   const PassOp<1>& op = dp->op;
-  // warps without a group (states below 5 qubits) leave the FP64 pipe's conversions
-  // of the operator to the others: 3 qubits, double-float dense 9.8 -> 7.9 us
-  if (!kSuper && (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= 1ull << (2 * n - 2)) return;
+  // double-float: warps without a group (states below 5 qubits) leave the FP64 pipe's
+  // conversions of the operator to the others: 3 qubits, dense 9.8 -> 7.9 us
+  if (std::is_same<T, df64>::value && !kSuper && (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u) >= 1ull << (2 * n - 2)) return;
   // the operator, uniform over the grid (a few dozen bytes from L1)
   T ur[4], ui[4], vr[4], vi[4], fr[4], fi[4];
   int src[2], srcb[2], fk[4];
